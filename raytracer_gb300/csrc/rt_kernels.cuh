@@ -67,7 +67,7 @@ struct Wave {
 // One work item of a multi-scene batch (rt_internal_render_multi): whole
 // tiles of one job with every sample of their pixels.  The batch's path
 // slots are the items' slots one after another; within an item, slot
-// path0 + s * npix + q is sample s of the item's pixel q, as in a
+// path0 + q * spp + s is sample s of the item's pixel q, as in a
 // single-scene batch.
 struct MultiItem {
     int job;             // scene-table index
