@@ -62,17 +62,41 @@ __device__ __forceinline__ float4 f4c(C3 c, float w) { return make_float4(c.r, c
 __device__ __forceinline__ V3 xyz(float4 a) { return v3(a.x, a.y, a.z); }
 __device__ __forceinline__ C3 rgb(float4 a) { return c3(a.x, a.y, a.z); }
 
-// warp-aggregated append to a queue
-__device__ __forceinline__ void q_push(int *queue, int *count, int value, bool pred)
+// Append `value` to queue k for every bit k set in `want`, by all 32 lanes of
+// a warp at once.  One atomic instruction serves the N queues (lane k adds for
+// queue k), so the warp waits for one round trip instead of one per queue.
+template <int N>
+__device__ __forceinline__ void q_push(int *const (&queue)[N], int *const (&count)[N], int value, unsigned want)
 {
-    unsigned mask = __ballot_sync(__activemask(), pred);
-    if (!pred) return;
-    int lane = threadIdx.x & 31;
-    int leader = __ffs(mask) - 1;
+    const int lane = threadIdx.x & 31;
+    unsigned mask[N], mine = 0;
+    int *cp = count[0];
+#pragma unroll
+    for (int k = 0; k < N; k++) {
+        mask[k] = __ballot_sync(0xffffffffu, (want >> k) & 1u);
+        if (lane == k) { mine = mask[k]; cp = count[k]; }
+    }
     int base = 0;
-    if (lane == leader) base = atomicAdd(count, __popc(mask));
-    base = __shfl_sync(mask, base, leader);
-    queue[base + __popc(mask & ((1u << lane) - 1))] = value;
+    if (mine) base = atomicAdd(cp, __popc(mine));
+#pragma unroll
+    for (int k = 0; k < N; k++) {
+        const int b = __shfl_sync(0xffffffffu, base, k);
+        if ((want >> k) & 1u) queue[k][b + __popc(mask[k] & ((1u << lane) - 1))] = value;
+    }
+}
+
+// The same for the shading and finish queues, each lane's slot to queue `t`
+// (negative: none), by all 32 lanes: one atomic instruction, a lane per queue
+// that occurs.
+__device__ __forceinline__ void q_push_class(const Wave &W, RoundCounters *C, int slot, int t)
+{
+    const int lane = threadIdx.x & 31;
+    const unsigned same = __match_any_sync(0xffffffffu, t);
+    const int leader = __ffs(same) - 1;
+    int base = 0;
+    if (t >= 0 && lane == leader) base = atomicAdd(&C->mat[t], __popc(same));
+    base = __shfl_sync(0xffffffffu, base, leader);
+    if (t >= 0) W.q_mat[t][base + __popc(same & ((1u << lane) - 1))] = slot;
 }
 
 // Film footprint of a sample inside its tile: Screen::addSample with the
@@ -238,23 +262,39 @@ __global__ void k_camera_multi(RenderParams P)
     }
 }
 
-// Sort a traced path by what its ray hit: the shading queue of the hit
-// surface's BSDF type, or the finish queue for a miss or a surface without a
-// BSDF.  Called by the lanes that just finished a closest-hit ray.
-// `n` is the round's closest-hit ray count: below P.sort_threshold the hits
-// are not sorted by material (one queue, one generic shading kernel).
-__device__ __forceinline__ void classify_hit(const RenderParams &P, const DevScene &S, RoundCounters *C, int slot,
-                                             int prim, int n)
+// The queue a traced path goes to by what its ray hit: the shading queue of
+// the hit surface's BSDF type, or the finish queue for a miss or a surface
+// without a BSDF.  `n` is the round's closest-hit ray count: below
+// P.sort_threshold the hits are not sorted by material (one queue, one
+// generic shading kernel).
+__device__ __forceinline__ int hit_queue(const RenderParams &P, const DevScene &S, int prim, int n)
 {
     const int t = prim == -1 ? -1 : prim_type(S, prim);
-    if (n < P.sort_threshold) {
-        q_push(P.W.q_mixed, &C->mixed, slot, t >= 0);
-    } else {
-#pragma unroll
-        for (int k = 0; k < RT_NBSDF; k++) q_push(P.W.q_mat[k], &C->mat[k], slot, t == k);
-        if (S.has_mixed) q_push(P.W.q_mixed, &C->mixed, slot, t == RT_QUEUE_MIXED);
-    }
-    q_push(P.W.q_fin, &C->fin, slot, t < 0);
+    return t < 0 ? RT_QUEUE_FIN : n < P.sort_threshold ? RT_QUEUE_MIXED : t;
+}
+
+// The next ray for each lane with `want`: its slot and its ray, or -1 when
+// the queue is empty.  One atomic per call.  (Reserving 32 entries at a time
+// and staging their rays in shared memory was slower, 23.1 against 21.2 ms of
+// closest-hit traversal on the 1.31M-triangle frame: the staging code spills
+// in the node loop, and the few lanes that fetch do not wait on the atomic
+// for long.)
+template <bool ANY>
+__device__ __forceinline__ int trace_fetch(const Wave &W, const int *queue, int *wc, int n, bool want, float4 &o, float4 &d)
+{
+    const int lane = threadIdx.x & 31;
+    const unsigned m = __ballot_sync(0xffffffffu, want);
+    if (!m) return -1;
+    const int leader = __ffs(m) - 1;
+    int base = 0;
+    if (lane == leader) base = atomicAdd(wc, __popc(m));
+    base = __shfl_sync(0xffffffffu, base, leader);
+    const int q = base + __popc(m & ((1u << lane) - 1));
+    if (!want || q >= n) return -1;
+    const int slot = queue[q];
+    o = ANY ? W.sh_o[slot] : W.ray_o[slot];
+    d = ANY ? W.sh_d[slot] : W.ray_d[slot];
+    return slot;
 }
 
 // ---------------------------------------------------------------- ray reordering
@@ -425,26 +465,17 @@ __global__ void __launch_bounds__(128, RT_TRACE_MINB) k_trace(RenderParams P, in
     for (;;) {
         // ---- fetch rays for lanes whose ray is finished
         const bool terminated = (node == RT_SENT);
-        const unsigned mterm = __ballot_sync(0xffffffffu, terminated);
-        const int nterm = __popc(mterm);
-        int base = 0;
-        if (nterm) {
-            const int leader = __ffs(mterm) - 1;
-            if (lane == leader) base = atomicAdd(wc, nterm);
-            base = __shfl_sync(0xffffffffu, base, leader);
-        }
+        float4 o4, d4;
+        const int got = trace_fetch<ANY>(P.W, queue, wc, n, terminated, o4, d4);
         if (terminated) {
-            int q = base + __popc(mterm & ((1u << lane) - 1));
-            has_ray = q < n;
+            has_ray = got >= 0;
             if (has_ray) {
-                slot = queue[q];
+                slot = got;
                 if (MULTI) {
                     ms = &P.scenes[P.W.sid[slot]];
                     mnodes = ms->nodes;
                     mtris = ms->tri_slots;
                 }
-                float4 o4 = ANY ? P.W.sh_o[slot] : P.W.ray_o[slot];
-                float4 d4 = ANY ? P.W.sh_d[slot] : P.W.ray_d[slot];
                 ox = o4.x; oy = o4.y; oz = o4.z; dx = d4.x; dy = d4.y; dz = d4.z;
                 tmin = adapt_mint(v3(ox, oy, oz), o4.w);
                 hit_t = d4.w;
@@ -519,6 +550,7 @@ __global__ void __launch_bounds__(128, RT_TRACE_MINB) k_trace(RenderParams P, in
             if (__popc(__activemask()) < RT_FETCH_THRESHOLD) break;
         }
         // ---- finished rays: analytic spheres, then store
+        int to_queue = -1;
         if (node == RT_SENT && has_ray) {
             if (!(ANY && hprim >= 0)) {
                 const int nsph = MULTI ? ms->n_spheres : S.n_spheres;
@@ -534,11 +566,11 @@ __global__ void __launch_bounds__(128, RT_TRACE_MINB) k_trace(RenderParams P, in
             if (ANY) P.W.occl[slot] = hprim != -1 ? 1 : 0;
             else {
                 P.W.hit[slot] = make_float4(hit_t, hu, hv, __int_as_float(hprim));
-                if (MULTI) classify_hit(P, *ms, C, slot, hprim, n);
-                else classify_hit(P, S, C, slot, hprim, n);
+                to_queue = MULTI ? hit_queue(P, *ms, hprim, n) : hit_queue(P, S, hprim, n);
             }
             has_ray = false;
         }
+        if (!ANY && __any_sync(0xffffffffu, to_queue >= 0)) q_push_class(P.W, C, slot, to_queue);
     }
     if (COUNT) {
         for (int off = 16; off > 0; off >>= 1) {
@@ -619,21 +651,12 @@ __global__ void __launch_bounds__(128, RT_TRACE4_MINB) k_trace4(RenderParams P, 
     for (;;) {
         // ---- fetch rays for lanes whose ray is finished
         const bool terminated = (node == RT_SENT);
-        const unsigned mterm = __ballot_sync(0xffffffffu, terminated);
-        const int nterm = __popc(mterm);
-        int base = 0;
-        if (nterm) {
-            const int leader = __ffs(mterm) - 1;
-            if (lane == leader) base = atomicAdd(wc, nterm);
-            base = __shfl_sync(0xffffffffu, base, leader);
-        }
+        float4 o4, d4;
+        const int got = trace_fetch<ANY>(P.W, queue, wc, n, terminated, o4, d4);
         if (terminated) {
-            int q = base + __popc(mterm & ((1u << lane) - 1));
-            has_ray = q < n;
+            has_ray = got >= 0;
             if (has_ray) {
-                slot = queue[q];
-                float4 o4 = ANY ? P.W.sh_o[slot] : P.W.ray_o[slot];
-                float4 d4 = ANY ? P.W.sh_d[slot] : P.W.ray_d[slot];
+                slot = got;
                 ox = o4.x; oy = o4.y; oz = o4.z; dx = d4.x; dy = d4.y; dz = d4.z;
                 tmin = adapt_mint(v3(ox, oy, oz), o4.w);
                 hit_t = d4.w;
@@ -711,6 +734,7 @@ __global__ void __launch_bounds__(128, RT_TRACE4_MINB) k_trace4(RenderParams P, 
             if (__popc(__activemask()) < RT_FETCH_THRESHOLD) break;
         }
         // ---- finished rays: analytic spheres, then store
+        int to_queue = -1;
         if (node == RT_SENT && has_ray) {
             if (!(ANY && hprim >= 0)) {
                 for (int si = 0; si < S.n_spheres; si++) {
@@ -724,10 +748,11 @@ __global__ void __launch_bounds__(128, RT_TRACE4_MINB) k_trace4(RenderParams P, 
             if (ANY) P.W.occl[slot] = hprim != -1 ? 1 : 0;
             else {
                 P.W.hit[slot] = make_float4(hit_t, hu, hv, __int_as_float(hprim));
-                classify_hit(P, S, C, slot, hprim, n);
+                to_queue = hit_queue(P, S, hprim, n);
             }
             has_ray = false;
         }
+        if (!ANY && __any_sync(0xffffffffu, to_queue >= 0)) q_push_class(P.W, C, slot, to_queue);
     }
     if (COUNT) {
         for (int off = 16; off > 0; off >>= 1) {
@@ -797,22 +822,13 @@ __global__ void __launch_bounds__(128, 8) k_trace8(RenderParams P, int round)
     for (;;) {
         // ---- fetch rays for lanes whose ray is finished
         const bool idle = !trav;
-        const unsigned midle = __ballot_sync(0xffffffffu, idle);
-        const int nidle = __popc(midle);
-        int base = 0;
         bool has_ray = trav;
-        if (nidle) {
-            const int leader = __ffs(midle) - 1;
-            if (lane == leader) base = atomicAdd(wc, nidle);
-            base = __shfl_sync(0xffffffffu, base, leader);
-        }
+        float4 o4, d4;
+        const int got = trace_fetch<ANY>(P.W, queue, wc, n, idle, o4, d4);
         if (idle) {
-            int q = base + __popc(midle & ((1u << lane) - 1));
-            has_ray = q < n;
+            has_ray = got >= 0;
             if (has_ray) {
-                slot = queue[q];
-                float4 o4 = ANY ? P.W.sh_o[slot] : P.W.ray_o[slot];
-                float4 d4 = ANY ? P.W.sh_d[slot] : P.W.ray_d[slot];
+                slot = got;
                 ox = o4.x; oy = o4.y; oz = o4.z; dx = d4.x; dy = d4.y; dz = d4.z;
                 tmin = adapt_mint(v3(ox, oy, oz), o4.w);
                 hit_t = d4.w;
@@ -921,6 +937,7 @@ __global__ void __launch_bounds__(128, 8) k_trace8(RenderParams P, int round)
             }
             if (__popc(__activemask()) < RT_FETCH_THRESHOLD) break;
         }
+        int to_queue = -1;
         if (!trav && has_ray) {
             if (!(ANY && hprim >= 0)) {
                 for (int si = 0; si < S.n_spheres; si++) {
@@ -934,10 +951,11 @@ __global__ void __launch_bounds__(128, 8) k_trace8(RenderParams P, int round)
             if (ANY) P.W.occl[slot] = hprim != -1 ? 1 : 0;
             else {
                 P.W.hit[slot] = make_float4(hit_t, hu, hv, __int_as_float(hprim));
-                classify_hit(P, S, C, slot, hprim, n);
+                to_queue = hit_queue(P, S, hprim, n);
             }
             has_ray = false;
         }
+        if (!ANY && __any_sync(0xffffffffu, to_queue >= 0)) q_push_class(P.W, C, slot, to_queue);
     }
     if (COUNT) {
         for (int off = 16; off > 0; off >>= 1) {
@@ -1053,9 +1071,9 @@ __global__ void __launch_bounds__(128) k_pt_finish(RenderParams P, int round)
 {
     round = cur_round(P, round);
     RoundCounters *C = &P.W.cnt[round];
-    const int nf = C->fin, n = nf + C->end;
+    const int nf = C->mat[RT_QUEUE_FIN], n = nf + C->end;
     for (int idx = blockIdx.x * blockDim.x + threadIdx.x; idx < n; idx += gridDim.x * blockDim.x) {
-        const int slot = idx < nf ? P.W.q_fin[idx] : P.W.q_end[idx - nf];
+        const int slot = idx < nf ? P.W.q_mat[RT_QUEUE_FIN][idx] : P.W.q_end[idx - nf];
         if (MULTI) pt_finish_path(P, P.scenes[P.W.sid[slot]], slot);
         else pt_finish_path(P, P.S, slot);
     }
@@ -1291,8 +1309,10 @@ __global__ void __launch_bounds__(128, RT_SHADE_MINB) k_pt_shade(RenderParams P,
     round = cur_round(P, round);
     RoundCounters *C = &P.W.cnt[round];
     RoundCounters *Cout = &P.W.cnt[round + 1];
-    const int n = BT == RT_QUEUE_MIXED ? C->mixed : C->mat[BT];
-    const int *qin = BT == RT_QUEUE_MIXED ? P.W.q_mixed : P.W.q_mat[BT];
+    const int n = C->mat[BT];
+    const int *qin = P.W.q_mat[BT];
+    int *const out_q[3] = {P.W.q_closest, P.W.q_shadow, P.W.q_end};
+    int *const out_n[3] = {&Cout->closest, &Cout->shadow, &Cout->end};
     int idx = blockIdx.x * blockDim.x + threadIdx.x;
     int stride = gridDim.x * blockDim.x;
     int iters = (n + stride - 1) / stride;
@@ -1304,9 +1324,7 @@ __global__ void __launch_bounds__(128, RT_SHADE_MINB) k_pt_shade(RenderParams P,
             if (MULTI) pt_shade_path<BT, ALL>(P, P.scenes[P.W.sid[slot]], slot, push_end, push_closest, push_shadow);
             else pt_shade_path<BT, ALL>(P, P.S, slot, push_end, push_closest, push_shadow);
         }
-        q_push(P.W.q_end, &Cout->end, slot, push_end);
-        q_push(P.W.q_closest, &Cout->closest, slot, push_closest);
-        q_push(P.W.q_shadow, &Cout->shadow, slot, push_shadow);
+        q_push(out_q, out_n, slot, (push_closest ? 1u : 0u) | (push_shadow ? 2u : 0u) | (push_end ? 4u : 0u));
     }
 }
 
@@ -2932,7 +2950,7 @@ extern "C" int64_t rt_path_state_bytes(int32_t integrator)
                          10 * sizeof(float4) +                 // tp rad ray_o ray_d hit bs nee sh_o sh_d out
                          3 * sizeof(int) +                     // rel_eta flags occl
                          2 +                                   // splat pix_irregular
-                         (4 + RT_NBSDF + 1) * sizeof(int) +    // fin end closest shadow, material, mixed queues
+                         (3 + RT_NQUEUE) * sizeof(int) +       // end closest shadow, shading and finish queues
                          3 * sizeof(int);                      // sid, sort keys and scratch
     return wave + (volpath ? 6 * (int64_t)sizeof(float4) : 0);   // v_seg v_p v_li0 v_li1 v_li2 v_val
 }
@@ -2966,12 +2984,10 @@ static rt_status ensure_wave(rt_ctx *c, int capacity, int max_rounds)
     ok &= alloc((void **)&W.out, P * sizeof(float4));
     ok &= alloc((void **)&W.splat, P);
     ok &= alloc((void **)&W.pix_irregular, P);
-    ok &= alloc((void **)&W.q_fin, P * sizeof(int));
     ok &= alloc((void **)&W.q_end, P * sizeof(int));
     ok &= alloc((void **)&W.q_closest, P * sizeof(int));
     ok &= alloc((void **)&W.q_shadow, P * sizeof(int));
-    for (int t = 0; t < RT_NBSDF; t++) ok &= alloc((void **)&W.q_mat[t], P * sizeof(int));
-    ok &= alloc((void **)&W.q_mixed, P * sizeof(int));
+    for (int t = 0; t < RT_NQUEUE; t++) ok &= alloc((void **)&W.q_mat[t], P * sizeof(int));
     ok &= alloc((void **)&W.cnt, (size_t)(max_rounds + 2) * sizeof(RoundCounters));
     ok &= alloc((void **)&W.sid, P * sizeof(int));
     ok &= alloc((void **)&W.sort_keys, P * sizeof(unsigned));
@@ -4055,13 +4071,13 @@ extern "C" rt_status rt_render_tile_static(rt_ctx *ctx, rt_scene *sc, const rt_r
     W.out = (float4 *)take(P * sizeof(float4));
     W.splat = (uint8_t *)take(P);
     W.pix_irregular = (uint8_t *)take((size_t)npix);
-    W.q_fin = (int *)take(P * sizeof(int));
+    W.q_mat[RT_QUEUE_FIN] = (int *)take(P * sizeof(int));
     W.q_end = (int *)take(P * sizeof(int));
     W.q_closest = (int *)take(P * sizeof(int));
     W.q_shadow = (int *)take(P * sizeof(int));
     for (int t = 0; t < RT_NBSDF; t++) W.q_mat[t] = (int *)take(P * sizeof(int));
     // textured and Microfacet BSDFs shade from the mixed queue
-    if (sc->S.has_mixed) W.q_mixed = (int *)take(P * sizeof(int));
+    if (sc->S.has_mixed) W.q_mat[RT_QUEUE_MIXED] = (int *)take(P * sizeof(int));
     W.cnt = (RoundCounters *)take((size_t)(rounds + 2) * sizeof(RoundCounters));
     W.capacity = (int)P;
     W.max_rounds = rounds;

@@ -13,13 +13,13 @@ enum { F_FIRST = 1, F_DELTA = 2, F_NEE = 4, F_END = 8, F_DONE = 16 };
 #define RT_NBSDF 6        // sorted shading queues (bsdf_queue): types 0-4, then the delta types;
                           // RT_QUEUE_MIXED (rt_device.cuh) is one more: textured BSDFs, and
                           // every BSDF in bounces below the sort threshold
+#define RT_QUEUE_FIN 7    // paths whose traced ray missed or hit a surface without a BSDF
+#define RT_NQUEUE 8
 
 struct RoundCounters {   // one per wavefront round, zeroed per batch
     int closest, shadow, wc_closest, wc_shadow;
-    int mat[RT_NBSDF];   // paths to shade per shading queue (material-sorted)
-    int fin;             // paths whose traced ray missed or hit a surface without a BSDF
+    int mat[RT_NQUEUE];  // paths per shading queue (material-sorted), in the mixed queue, to finish
     int end;             // paths that ended in shading with a light sample pending
-    int mixed;           // paths to shade, not sorted by material (round below the sort threshold)
     int pad[3];
 };
 
@@ -42,9 +42,8 @@ struct Wave {
     uint8_t *pix_irregular;  // per batch pixel: some sample splats off its pixel
     // queues of the current round
     int *q_closest, *q_shadow;
-    int *q_mat[RT_NBSDF];  // shading queues (bsdf_queue), filled by the closest-hit trace
-    int *q_mixed;          // the unsorted shading queue (RT_QUEUE_MIXED)
-    int *q_fin;        // rays that missed or hit a surface without a BSDF (to finish)
+    int *q_mat[RT_NQUEUE];  // shading queues (bsdf_queue), the unsorted one (RT_QUEUE_MIXED) and the
+                            // paths to finish (RT_QUEUE_FIN), filled by the closest-hit trace
     int *q_end;        // paths whose BSDF sample was zero, light sample pending
     // ray reordering (optional): per-ray keys, the reordered queue, key counts
     unsigned *sort_keys;

@@ -440,10 +440,13 @@ __device__ __noinline__ C3 vw_tr_sampled(const DevScene &S, Ray ray, Pcg32 &rng,
 #ifndef RT_VW_MINB_TRSAMP
 #define RT_VW_MINB_TRSAMP RT_VW_MINB
 #endif
+// whole warps run every pass of the loop (VW_LIVE: the lane has a path), so
+// that the pushes at its end are the warp's
 #define VW_LOOP(COUNT, QUEUE)                                                                      \
     const int n_ = (COUNT);                                                                        \
     const int *qin_ = (QUEUE);                                                                     \
-    for (int i_ = blockIdx.x * blockDim.x + threadIdx.x; i_ < n_; i_ += gridDim.x * blockDim.x)
+    for (int i_ = blockIdx.x * blockDim.x + threadIdx.x; (i_ & ~31) < n_; i_ += gridDim.x * blockDim.x)
+#define VW_LIVE (i_ < n_)
 
 // The trace queue of a round: rounds alternate between two arrays, since
 // the kernel that reads round r's queue also appends to round r + 1's.
@@ -467,9 +470,13 @@ __global__ void __launch_bounds__(128, RT_VW_MINB_STEP) k_vw_trace_step(RenderPa
     RoundCounters *Cn = &P.W.cnt[round + 1];
     int *next_q = vw_trace_queue(P, round + 1);
     int limit = 0;
+    int *const out_q[4] = {P.W.q_shadow, P.W.q_mat[1], P.W.q_mat[4], next_q};
+    int *const out_n[4] = {&C->shadow, &C->mat[1], &C->mat[4], &Cn->closest};
     VW_LOOP(C->closest, vw_trace_queue(P, round))
     {
-        const int slot = qin_[i_];
+        const int slot = VW_LIVE ? qin_[i_] : 0;
+        unsigned want = 0;
+        if (VW_LIVE) {
         // ---- the trace (k_vw_trace)
         int flags = P.W.flags[slot];
         const float4 ro = P.W.ray_o[slot], rd = P.W.ray_d[slot];
@@ -575,11 +582,9 @@ __global__ void __launch_bounds__(128, RT_VW_MINB_STEP) k_vw_trace_step(RenderPa
                 P.W.flags[slot] = (flags & ((1 << VF_GUARD_SHIFT) - 1)) | (guard << VF_GUARD_SHIFT);
             }
         }
-        const bool scat = (flags & VF_SCAT) != 0;
-        q_push(P.W.q_shadow, &C->shadow, slot, push_shadow);
-        q_push(P.W.q_mat[1], &C->mat[1], slot, push_sample && scat);
-        q_push(P.W.q_mat[4], &C->mat[4], slot, push_sample && !scat);
-        q_push(next_q, &Cn->closest, slot, push_trace);
+        want = push_shadow ? 1u : push_sample ? ((flags & VF_SCAT) ? 2u : 4u) : push_trace ? 8u : 0u;
+        }
+        q_push(out_q, out_n, slot, want);
     }
     if (limit) atomicOr(P.limit_flag, RT_LIM_VOLPATH);
 }
@@ -590,9 +595,13 @@ __global__ void __launch_bounds__(128, RT_VW_MINB_SHADOW) k_vw_shadow(RenderPara
     const DevScene &S = P.S;
     RoundCounters *C = &P.W.cnt[round];
     int limit = 0;
+    int *const out_q[2] = {P.W.q_mat[1], P.W.q_mat[4]};
+    int *const out_n[2] = {&C->mat[1], &C->mat[4]};
     VW_LOOP(C->shadow, P.W.q_shadow)
     {
-        const int slot = qin_[i_];
+        const int slot = VW_LIVE ? qin_[i_] : 0;
+        unsigned want = 0;
+        if (VW_LIVE) {
         Pcg32 rng = P.W.rng[slot];
         float4 pv = P.W.v_p[slot], l0 = P.W.v_li0[slot], l1 = P.W.v_li1[slot], iv = P.W.v_val[slot];
         const int medium = __float_as_int(P.W.v_seg[slot].w);
@@ -604,8 +613,9 @@ __global__ void __launch_bounds__(128, RT_VW_MINB_SHADOW) k_vw_shadow(RenderPara
         P.W.rng[slot] = rng;
         const int flags = P.W.flags[slot] | VF_HASVAL;
         P.W.flags[slot] = flags;
-        q_push(P.W.q_mat[1], &C->mat[1], slot, (flags & VF_SCAT) != 0);
-        q_push(P.W.q_mat[4], &C->mat[4], slot, (flags & VF_SCAT) == 0);
+        want = (flags & VF_SCAT) ? 1u : 2u;
+        }
+        q_push(out_q, out_n, slot, want);
     }
     if (limit) atomicOr(P.limit_flag, RT_LIM_VOLPATH);
 }
@@ -619,9 +629,13 @@ __global__ void __launch_bounds__(128, RT_VW_MINB_SAMPLE) k_vw_sample_surface(Re
     round = cur_round(P, round);
     const DevScene &S = P.S;
     RoundCounters *C = &P.W.cnt[round];
+    int *const out_q[1] = {P.W.q_mat[2]};
+    int *const out_n[1] = {&C->mat[2]};
     VW_LOOP(C->mat[4], P.W.q_mat[4])
     {
-        const int slot = qin_[i_];
+        const int slot = VW_LIVE ? qin_[i_] : 0;
+        unsigned want = 0;
+        if (VW_LIVE) {
         int flags = P.W.flags[slot];
         Pcg32 rng = P.W.rng[slot];
         float4 radv = P.W.rad[slot], tpv = P.W.tp[slot];
@@ -679,7 +693,9 @@ __global__ void __launch_bounds__(128, RT_VW_MINB_SAMPLE) k_vw_sample_surface(Re
             P.W.v_seg[slot] = make_float4(seg.x, seg.y, seg.z, __int_as_float(medium));
             P.W.flags[slot] = flags;
         }
-        q_push(P.W.q_mat[2], &C->mat[2], slot, push);
+        want = push ? 1u : 0u;
+        }
+        q_push(out_q, out_n, slot, want);
     }
 }
 
@@ -687,10 +703,10 @@ __global__ void __launch_bounds__(128, RT_VW_MINB_SAMPLE) k_vw_sample_surface(Re
 // MIS of what the ray found, throughput, Russian roulette
 // (VolPathTracing.cpp:300-367).  ro, rd: the sampled ray; h, seg, was,
 // flags: what evalTransmittanceFromSampledBSDF reported; L: the radiance with
-// this vertex's light-sample MIS.  Survivors go to the next round's trace
-// queue with their sampled ray.
-__device__ __forceinline__ void vw_finish_one(const RenderParams &P, const DevScene &S, RoundCounters *Cn,
-                                              int *next_q, int slot, int flags, Pcg32 rng, float4 ro, float4 rd,
+// this vertex's light-sample MIS.  Returns whether the path goes on (to the
+// next round's trace queue, with its sampled ray).
+__device__ __forceinline__ bool vw_finish_one(const RenderParams &P, const DevScene &S, int slot, int flags, Pcg32 rng,
+                                              float4 ro, float4 rd,
                                               float4 seg, const Hit &h, bool was, C3 tr, C3 L, int depth,
                                               float4 tpv, float4 bsv)
 {
@@ -758,7 +774,7 @@ __device__ __forceinline__ void vw_finish_one(const RenderParams &P, const DevSc
         P.W.rad[slot] = f4c(L, __int_as_float(depth));
         P.W.tp[slot] = f4c(T, eta);
     }
-    q_push(next_q, &Cn->closest, slot, !done);
+    return !done;
 }
 
 // k_vw_trsamp_finish: evalTransmittanceFromSampledBSDF along the ray that
@@ -771,9 +787,13 @@ __global__ void __launch_bounds__(128, RT_VW_MINB_TRSAMP) k_vw_trsamp_finish(Ren
     RoundCounters *Cn = &P.W.cnt[round + 1];
     int *next_q = vw_trace_queue(P, round + 1);
     int limit = 0;
+    int *const out_q[1] = {next_q};
+    int *const out_n[1] = {&Cn->closest};
     VW_LOOP(C->mat[2], P.W.q_mat[2])
     {
-        const int slot = qin_[i_];
+        const int slot = VW_LIVE ? qin_[i_] : 0;
+        unsigned want = 0;
+        if (VW_LIVE) {
         int flags = P.W.flags[slot];
         Pcg32 rng = P.W.rng[slot];
         const float4 ro = P.W.ray_o[slot], rd = P.W.ray_d[slot];
@@ -788,8 +808,12 @@ __global__ void __launch_bounds__(128, RT_VW_MINB_TRSAMP) k_vw_trsamp_finish(Ren
         flags = (flags & ~(VF_WAS | VF_NEWM)) | (was ? VF_WAS : 0) | (newm >= 0 ? VF_NEWM : 0);
         seg = make_float4(so.x, so.y, so.z, seg.w);
         const float4 radv = P.W.rad[slot];
-        vw_finish_one(P, S, Cn, next_q, slot, flags, rng, ro, rd, seg, h, was, tr, rgb(radv),
-                      __float_as_int(radv.w), P.W.tp[slot], P.W.bs[slot]);
+        want = vw_finish_one(P, S, slot, flags, rng, ro, rd, seg, h, was, tr, rgb(radv), __float_as_int(radv.w),
+                             P.W.tp[slot], P.W.bs[slot])
+                   ? 1u
+                   : 0u;
+        }
+        q_push(out_q, out_n, slot, want);
     }
     if (limit) atomicOr(P.limit_flag, RT_LIM_VOLPATH);
 }
@@ -807,9 +831,13 @@ __global__ void __launch_bounds__(128, RT_VW_MINB_TRSAMP) k_vw_scatter(RenderPar
     RoundCounters *Cn = &P.W.cnt[round + 1];
     int *next_q = vw_trace_queue(P, round + 1);
     int limit = 0;
+    int *const out_q[1] = {next_q};
+    int *const out_n[1] = {&Cn->closest};
     VW_LOOP(C->mat[1], P.W.q_mat[1])
     {
-        const int slot = qin_[i_];
+        const int slot = VW_LIVE ? qin_[i_] : 0;
+        unsigned want = 0;
+        if (VW_LIVE) {
         int flags = P.W.flags[slot];
         Pcg32 rng = P.W.rng[slot];
         float4 seg = P.W.v_seg[slot];
@@ -844,8 +872,12 @@ __global__ void __launch_bounds__(128, RT_VW_MINB_TRSAMP) k_vw_scatter(RenderPar
                 L = L + ((rgb(tpv) * value) * ev) * w;
             }
         }
-        vw_finish_one(P, S, Cn, next_q, slot, flags, rng, ro, rd, seg, h, was, tr, L, __float_as_int(radv.w), tpv,
-                      f4c(cfill(pfw), pfpdf));
+        want = vw_finish_one(P, S, slot, flags, rng, ro, rd, seg, h, was, tr, L, __float_as_int(radv.w), tpv,
+                             f4c(cfill(pfw), pfpdf))
+                   ? 1u
+                   : 0u;
+        }
+        q_push(out_q, out_n, slot, want);
     }
     if (limit) atomicOr(P.limit_flag, RT_LIM_VOLPATH);
 }
