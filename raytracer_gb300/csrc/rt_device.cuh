@@ -1708,83 +1708,113 @@ __device__ __forceinline__ C3 homog_tr(const DevMedium &m, float mint, float max
     float t = maxt - mint;
     return c3(expf(-m.sigma_t[0] * t), expf(-m.sigma_t[1] * t), expf(-m.sigma_t[2] * t));
 }
-// GridVolume::lookupSigmaT (volume/GridVolume.cpp:118-149) * scale
-__device__ __forceinline__ float grid_lookup(const DevMedium &m, V3 pa)
+#define RT_TRACK_CAP (1 << 20)
+
+// A grid medium's lookup fields in registers.  The tracking loops write their
+// path's stream state through a reference; read through the medium pointer,
+// the fields would be loaded again after every such write.
+struct GridView {
+    const float *density;
+    int nx, ny, nz;
+    float fx, fy, fz, scale, max_sigma_t;
+};
+__device__ __forceinline__ GridView grid_view(const DevMedium &m)
 {
-    float px = pa.x * (float)m.res[0], py = pa.y * (float)m.res[1], pz = pa.z * (float)m.res[2];
+    GridView g;
+    g.density = m.density;
+    g.nx = m.res[0]; g.ny = m.res[1]; g.nz = m.res[2];
+    g.fx = (float)g.nx; g.fy = (float)g.ny; g.fz = (float)g.nz;
+    g.scale = m.scale;
+    g.max_sigma_t = m.max_sigma_t;
+    return g;
+}
+// GridVolume::lookupSigmaT (volume/GridVolume.cpp:118-149) * scale
+__device__ __forceinline__ float grid_lookup(const GridView &g, V3 pa)
+{
+    float px = pa.x * g.fx, py = pa.y * g.fy, pz = pa.z * g.fz;
     float fx = floorf(px), fy = floorf(py), fz = floorf(pz);
     int ix = (int)fx, iy = (int)fy, iz = (int)fz;
-    if (ix < 0 || iy < 0 || iz < 0) return 0.0f * m.scale;
-    if (ix >= m.res[0] - 1 || iy >= m.res[1] - 1 || iz >= m.res[2] - 1) return 0.0f * m.scale;
-    size_t row = (size_t)m.res[0], slab = row * (size_t)m.res[1];
-    size_t off = (size_t)iz * slab + (size_t)iy * row + (size_t)ix;
-    const float *D = m.density;
-    float d000 = __ldg(D + off), d001 = __ldg(D + off + 1), d010 = __ldg(D + off + row),
-          d011 = __ldg(D + off + row + 1);
-    float d100 = __ldg(D + off + slab), d101 = __ldg(D + off + slab + 1), d110 = __ldg(D + off + slab + row),
-          d111 = __ldg(D + off + slab + row + 1);
+    if (ix < 0 || iy < 0 || iz < 0) return 0.0f * g.scale;
+    if (ix >= g.nx - 1 || iy >= g.ny - 1 || iz >= g.nz - 1) return 0.0f * g.scale;
+    size_t row = (size_t)g.nx, slab = row * (size_t)g.ny;
+    const float *D = g.density + ((size_t)iz * slab + (size_t)iy * row + (size_t)ix);
+    float d000 = __ldg(D), d001 = __ldg(D + 1), d010 = __ldg(D + row), d011 = __ldg(D + row + 1);
+    D += slab;
+    float d100 = __ldg(D), d101 = __ldg(D + 1), d110 = __ldg(D + row), d111 = __ldg(D + row + 1);
     float w1x = px - fx, w1y = py - fy, w1z = pz - fz;
     float w0x = 1 - w1x, w0y = 1 - w1y, w0z = 1 - w1z;
     float v = ((d000 * w0x + d001 * w1x) * w0y + (d010 * w0x + d011 * w1x) * w1y) * w0z +
               ((d100 * w0x + d101 * w1x) * w0y + (d110 * w0x + d111 * w1x) * w1y) * w1z;
-    return v * m.scale;
+    return v * g.scale;
 }
 
-#define RT_TRACK_CAP (1 << 20)
-
 // Heterogeneous::transmittance (medium/Heterogeneous.cpp:419-489): ratio tracking + RR
-__device__ __forceinline__ C3 hetero_tr(const DevMedium &m, Ray wr, Pcg32 &rng, int &limit)
+__device__ __forceinline__ C3 hetero_tr(const DevMedium &m, Ray wr, Pcg32 &rng_, int &limit)
 {
     V3 o = xf_point(m.world_to_array, wr.o), d = xf_vector(m.world_to_array, wr.d);
     float tmax = wr.maxt - wr.mint;
     float tr = 1.f, st;
-    int breaker = 0;
     float nearT, farT;
     const float bmin[3] = {0.f, 0.f, 0.f}, bmax[3] = {1.f, 1.f, 1.f};
     if (!ref_box_hit(bmin, bmax, o, d, wr.mint, wr.maxt, nearT, farT)) return cfill(1.f);
     tmax = smin(tmax, farT);
     st = smax(nearT, wr.mint);
-    for (;;) {
-        st += -logf(1.f - next1d(rng)) / m.max_sigma_t;
-        float proba = grid_lookup(m, o + st * d);
-        if (st >= tmax) return cfill(tr);
-        tr *= 1 - smax(0.f, proba / m.max_sigma_t);
+    const GridView g = grid_view(m);
+    Pcg32 rng = rng_;
+    // the reference gives up after 1026 lookups (its breaker); one past the
+    // end of the segment is not looked up here (it does not count)
+    for (int breaker = 0;; breaker++) {
+        st += -logf(1.f - next1d(rng)) / g.max_sigma_t;
+        if (st >= tmax) break;
+        const float proba = grid_lookup(g, o + st * d);
+        tr *= 1 - smax(0.f, proba / g.max_sigma_t);
         const float threshold = .1f;
         if (tr < threshold) {
             float q = smax(.05f, 1 - tr);
-            if (next1d(rng) < q) return cfill(0.f);
+            if (next1d(rng) < q) { tr = 0.f; break; }
             tr /= 1 - q;
         }
-        if (breaker > 1024) return cfill(0.f);
-        breaker++;
+        if (breaker > 1024) { tr = 0.f; break; }
     }
+    rng_ = rng;
+    return cfill(tr);
 }
 
 // Heterogeneous::sampleDistance (Heterogeneous.cpp:491-546): delta tracking
-__device__ __forceinline__ bool hetero_sample(const DevMedium &m, Ray wr, Pcg32 &rng, float &t, C3 &w, C3 &em,
+__device__ __forceinline__ bool hetero_sample(const DevMedium &m, Ray wr, Pcg32 &rng_, float &t_, C3 &w, C3 &em,
                                               int &limit)
 {
-    t = wr.mint;
+    float t = wr.mint;
     float cur = 0.f;
     float nearT, farT;
+    em = cfill(0.f);
     if (!ref_box_hit(m.wbox_min, m.wbox_max, wr.o, wr.d, wr.mint, wr.maxt, nearT, farT)) {
-        w = cfill(1.f); em = cfill(0.f); t = wr.maxt;
+        w = cfill(1.f); t_ = wr.maxt;
         return false;
     }
-    float tmax = smin(wr.maxt, farT);
-    int steps = 0;
-    for (;;) {
-        t += -logf(1.f - next1d(rng)) / m.max_sigma_t;
-        if (t > tmax) { w = cfill(1.f); em = cfill(0.f); t = tmax; return false; }
+    const float tmax = smin(wr.maxt, farT);
+    const GridView g = grid_view(m);
+    float M[16];
+#pragma unroll
+    for (int i = 0; i < 16; i++) M[i] = m.world_to_array[i];
+    Pcg32 rng = rng_;
+    bool in = true, capped = false;
+    for (int steps = 0;;) {
+        t += -logf(1.f - next1d(rng)) / g.max_sigma_t;
+        if (t > tmax) { in = false; t = tmax; break; }
         V3 pw = wr.o + t * wr.d;
-        cur = grid_lookup(m, xf_point(m.world_to_array, pw));
-        float proba = cur / m.max_sigma_t;
+        cur = grid_lookup(g, xf_point(M, pw));
+        float proba = cur / g.max_sigma_t;
         if (next1d(rng) < proba) break;
-        if (++steps >= RT_TRACK_CAP) { limit = 1; w = cfill(0.f); em = cfill(0.f); return true; }
+        if (++steps >= RT_TRACK_CAP) { capped = true; break; }
     }
-    if (cur != 0.f) w = cload(m.albedo); else w = cfill(0.f);
-    em = cfill(0.f);
-    return true;
+    rng_ = rng;
+    t_ = t;
+    if (capped) limit = 1;
+    if (!in) w = cfill(1.f);
+    else if (cur != 0.f && !capped) w = cload(m.albedo);
+    else w = cfill(0.f);
+    return in;
 }
 
 __device__ __forceinline__ bool medium_sample(const DevMedium &m, Ray r, Pcg32 &rng, float &t, C3 &w, C3 &em,
