@@ -1,6 +1,6 @@
 // rt_volpath.cuh -- VolPathTracing on the device: the persistent kernel
 // (k_volpath, one vol_step pass of the reference's bounce loop per call) and
-// the wavefront of six kernels over path queues (k_vw_*).  Textually part of
+// the wavefront of five kernels over path queues (k_vw_*).  Textually part of
 // rt_api.cu (included there after the PathTracingMIS kernels), which holds
 // RenderParams, the queue helpers and the BSDF dispatch these use.
 #pragma once
@@ -379,7 +379,7 @@ __device__ __forceinline__ bool vw_light_pick(const DevScene &S, V3 p, Pcg32 &rn
     if (S.n_lights == 0) return false;
     V2 u = next2d(rng);
     int idx = cdf_sample_reuse(S.light_cdf, S.n_lights + 1, u.x, lw);
-    vp_light_sample(S, idx, p, u, li);
+    light_sample(S, idx, p, u, li);
     return li.pdf > 0 && lum(li.intensity) > 0;
 }
 __device__ __forceinline__ void vw_store_light(const RenderParams &P, int slot, const LightRec &li, V3 p, float lw)
@@ -393,9 +393,11 @@ __device__ __forceinline__ void vw_store_light(const RenderParams &P, int slot, 
 __device__ __forceinline__ void vw_done(const RenderParams &P, int slot, C3 L) { P.W.out[slot] = f4c(L, 0.f); }
 
 // evalTransmittanceFromSampledBSDF (VolPathTracing.cpp:369-424), as
-// eval_tr_sampled, reporting the segment origin of the hit instead of its frame
-__device__ __noinline__ C3 vw_tr_sampled(const DevScene &S, Ray ray, Pcg32 &rng, int medium, Hit &h, V3 &seg, bool &was,
-                                         int &newm, int &limit)
+// eval_tr_sampled, reporting the segment origin of the hit instead of its
+// frame, and in h1 and was1 the hit of the ray's first segment: what the
+// trace of the same ray at the end of the pass would find
+__device__ __forceinline__ C3 vw_tr_sampled(const DevScene &S, Ray ray, Pcg32 &rng, int medium, Hit &h, V3 &seg, bool &was,
+                                         Hit &h1, bool &was1, int &newm, int &limit)
 {
     Ray tr = ray;
     C3 T = cfill(1.f);
@@ -403,10 +405,11 @@ __device__ __noinline__ C3 vw_tr_sampled(const DevScene &S, Ray ray, Pcg32 &rng,
     was = false;
     for (int guard = 0; guard < 4096; guard++) {
         Hit nh;
-        was = vp_trace(S, tr.o, tr.d, tr.mint, tr.maxt, nh);
+        was = trace_ray<false>(S, tr.o, tr.d, tr.mint, tr.maxt, nh);
         if (was) { h = nh; seg = tr.o; }
+        if (first) { h1 = h; was1 = was; }
         if (medium >= 0)
-            T = T * vp_medium_tr(S.media[medium], make_ray(tr.o, tr.d, first ? tr.mint : 0.f, was ? h.t : tr.maxt), rng, limit);
+            T = T * medium_tr(S.media[medium], make_ray(tr.o, tr.d, first ? tr.mint : 0.f, was ? h.t : tr.maxt), rng, limit);
         if (was && prim_bsdf(S, h.prim) >= 0) return T;
         first = false;
         if (!was || iszero(T)) return T;
@@ -414,7 +417,7 @@ __device__ __noinline__ C3 vw_tr_sampled(const DevScene &S, Ray ray, Pcg32 &rng,
         const V3 seg_o = tr.o;
         tr = make_ray(np, tr.d, RT_EPSILON, tr.maxt);
         if (prim_interior(S, h.prim) != prim_exterior(S, h.prim)) {
-            Frame f = vp_frame(S, h, seg_o, tr.d);
+            Frame f = hit_frame(S, h, seg_o, tr.d);
             medium = dot(f.n, tr.d) < 0.f ? prim_interior(S, h.prim) : prim_exterior(S, h.prim);
             newm = medium;
         }
@@ -423,10 +426,42 @@ __device__ __noinline__ C3 vw_tr_sampled(const DevScene &S, Ray ray, Pcg32 &rng,
     return T;
 }
 
+__device__ __forceinline__ C3 vw_transmittance(const DevScene &S, Ray ray, int medium, Pcg32 &rng, int &limit)
+{
+    Ray tr = ray;
+    C3 T = cfill(1.f);
+    float dist = ray.maxt;
+    bool first = true;
+    for (int guard = 0; guard < 4096; guard++) {
+        Hit h;
+        bool inter = trace_ray<false>(S, tr.o, tr.d, tr.mint, tr.maxt, h);
+        if (inter && prim_bsdf(S, h.prim) >= 0) return cfill(0.f);
+        if (inter) dist -= h.t;
+        if (medium >= 0)
+            T = T * medium_tr(S.media[medium], make_ray(tr.o, tr.d, first ? tr.mint : 0.f, inter ? h.t : dist), rng, limit);
+        first = false;
+        if (!inter || iszero(T)) return T;
+        V3 np = tr.o + h.t * tr.d;
+        Frame f = hit_frame(S, h, tr.o, tr.d);
+        tr = make_ray(np, tr.d, RT_EPSILON, dist);
+        if (prim_interior(S, h.prim) != prim_exterior(S, h.prim))
+            medium = dot(f.n, tr.d) < 0.f ? prim_interior(S, h.prim) : prim_exterior(S, h.prim);
+    }
+    limit = 1;
+    return cfill(0.f);
+}
+
+// Each wavefront kernel calls its traversal, tracking, frame and light code
+// from one place, so all of it is inline: the calls of the out-of-line copies
+// (the vp_ functions, which the persistent kernel shares among many places)
+// passed rays, hits and stream states through local memory and waited on
+// instruction fetch (7-10 cycles per issue).  128^3 grid-medium frame,
+// 512^2 x 128 spp: 61.5 ms with the calls, 51.7 ms inline, 50.4 ms with 6
+// blocks per SM (80 registers, hardly any spills) instead of 8.
 // resident 128-thread blocks per SM of each wavefront kernel (its launch
-// bound and its grid); the tracking loops of shadow and trsamp wait on memory
+// bound and its grid); 5 and 7 for any one of them were within 1 %
 #ifndef RT_VW_MINB
-#define RT_VW_MINB 8
+#define RT_VW_MINB 6
 #endif
 #ifndef RT_VW_MINB_STEP
 #define RT_VW_MINB_STEP RT_VW_MINB
@@ -462,6 +497,12 @@ __device__ __forceinline__ int *vw_trace_queue(const RenderParams &P, int round)
 // sample of sampleAttenuatedLightDirect.  The trace's hit, segment origin,
 // flags and depth stay in registers for the step; the hit is stored for the
 // kernels after it.
+// The reference traces a bounce's ray twice (VolPathTracing.cpp:105, :360).
+// The first segment of the sampled ray's transmittance is that same ray, with
+// the same bounds, and a trace draws no numbers, so the pass's last trace
+// takes its hit from there (vw_finish_one stores it); only camera rays and
+// the rays behind a null boundary are traced here.  They come first in the
+// queue, so few warps mix the two.  128^3 grid-medium frame: 64.4 -> 63.6 ms.
 __global__ void __launch_bounds__(128, RT_VW_MINB_STEP) k_vw_trace_step(RenderParams P, int round)
 {
     round = cur_round(P, round);
@@ -483,6 +524,7 @@ __global__ void __launch_bounds__(128, RT_VW_MINB_STEP) k_vw_trace_step(RenderPa
         float4 radv = P.W.rad[slot];
         float4 seg;
         Hit h;
+        const bool traces = (flags & (VF_FIRST | VF_NULLX)) != 0;
         if (flags & VF_FIRST) {
             h.t = RT_MAX_REAL; h.u = h.v = 0.f; h.prim = -1;
             seg = make_float4(0.f, 0.f, 0.f, __int_as_float(S.cam.medium));
@@ -496,16 +538,16 @@ __global__ void __launch_bounds__(128, RT_VW_MINB_STEP) k_vw_trace_step(RenderPa
                 radv.w = __int_as_float(__float_as_int(radv.w) + 1);
             }
         }
-        {
+        if (traces) {
             Hit nh;
-            const bool was = vp_trace(S, xyz(ro), xyz(rd), ro.w, rd.w, nh);
+            const bool was = trace_ray<false>(S, xyz(ro), xyz(rd), ro.w, rd.w, nh);
             if (was) {
                 h = nh;
                 seg = make_float4(ro.x, ro.y, ro.z, seg.w);
             }
             flags = (flags & ~(VF_NULLX | VF_WAS)) | (was ? VF_WAS : 0);
+            P.W.hit[slot] = make_float4(h.t, h.u, h.v, __int_as_float(h.prim));
         }
-        P.W.hit[slot] = make_float4(h.t, h.u, h.v, __int_as_float(h.prim));
         // ---- the step (k_vw_step)
         const float4 tpv = P.W.tp[slot];
         C3 L = rgb(radv), T = rgb(tpv);
@@ -525,20 +567,15 @@ __global__ void __launch_bounds__(128, RT_VW_MINB_STEP) k_vw_trace_step(RenderPa
             C3 wm = cfill(0.f), em = cfill(0.f);
             bool scattered = false;
             if (medium >= 0)
-                scattered = vp_medium_sample(S.media[medium], make_ray(ray.o, ray.d, ray.mint, h.t), rng, t, wm, em, limit);
-            bool done = false;
+                scattered = medium_sample(S.media[medium], make_ray(ray.o, ray.d, ray.mint, h.t), rng, t, wm, em, limit);
+            bool done = false, vertex = false;
+            V3 vp = v3(0.f, 0.f, 0.f);
             if (scattered) {
                 L = L + T * em;
                 T = T * wm;
-                V3 p = ray.o + t * ray.d;
-                LightRec li;
-                float lw;
-                const bool shadow = vw_light_pick(S, p, rng, li, lw);
-                vw_store_light(P, slot, li, p, lw);
+                vp = ray.o + t * ray.d;
                 flags |= VF_SCAT;
-                flags &= ~VF_HASVAL;
-                push_shadow = shadow;
-                push_sample = !shadow;
+                vertex = true;
             } else {
                 flags &= ~VF_SCAT;
                 if (medium >= 0) {
@@ -549,7 +586,7 @@ __global__ void __launch_bounds__(128, RT_VW_MINB_STEP) k_vw_trace_step(RenderPa
                     if ((flags & VF_EMISSION) && S.env_light >= 0) L = L + T * env_le(S.lights[S.env_light], ray.d);
                     done = true;
                 } else {
-                    Frame fr = vp_frame(S, h, xyz(seg), ray.d);
+                    Frame fr = hit_frame(S, h, xyz(seg), ray.d);
                     if (prim_bsdf(S, h.prim) < 0) {
                         // null boundary: through, without a bounce
                         ray = make_ray(fr.p, ray.d, RT_EPSILON, RT_MAX_REAL);
@@ -562,15 +599,18 @@ __global__ void __launch_bounds__(128, RT_VW_MINB_STEP) k_vw_trace_step(RenderPa
                     } else {
                         int hl = prim_light(S, h.prim);
                         if ((flags & VF_EMISSION) && hl >= 0) L = L + T * area_le(S, hl, -ray.d, fr.n);
-                        LightRec li;
-                        float lw;
-                        const bool shadow = vw_light_pick(S, fr.p, rng, li, lw);
-                        vw_store_light(P, slot, li, fr.p, lw);
-                        flags &= ~VF_HASVAL;
-                        push_shadow = shadow;
-                        push_sample = !shadow;
+                        vp = fr.p;
+                        vertex = true;
                     }
                 }
+            }
+            if (vertex) {
+                LightRec li;
+                float lw;
+                push_shadow = vw_light_pick(S, vp, rng, li, lw);
+                push_sample = !push_shadow;
+                vw_store_light(P, slot, li, vp, lw);
+                flags &= ~VF_HASVAL;
             }
             if (done) {
                 vw_done(P, slot, L);
@@ -605,7 +645,7 @@ __global__ void __launch_bounds__(128, RT_VW_MINB_SHADOW) k_vw_shadow(RenderPara
         Pcg32 rng = P.W.rng[slot];
         float4 pv = P.W.v_p[slot], l0 = P.W.v_li0[slot], l1 = P.W.v_li1[slot], iv = P.W.v_val[slot];
         const int medium = __float_as_int(P.W.v_seg[slot].w);
-        C3 tr = eval_transmittance(S, make_ray(xyz(pv), xyz(l0), RT_EPSILON, l0.w - RT_EPSILON), medium, rng, limit);
+        C3 tr = vw_transmittance(S, make_ray(xyz(pv), xyz(l0), RT_EPSILON, l0.w - RT_EPSILON), medium, rng, limit);
         float pdf = l1.w * pv.w;
         C3 value = (tr * rgb(iv)) / pdf;
         P.W.v_li1[slot] = make_float4(l1.x, l1.y, l1.z, pdf);
@@ -650,7 +690,7 @@ __global__ void __launch_bounds__(128, RT_VW_MINB_SAMPLE) k_vw_sample_surface(Re
         {
             float4 hv = P.W.hit[slot];
             Hit h; h.t = hv.x; h.u = hv.y; h.v = hv.z; h.prim = __float_as_int(hv.w);
-            Frame fr = vp_frame(S, h, xyz(seg), ray.d);
+            Frame fr = hit_frame(S, h, xyz(seg), ray.d);
             const DevBsdf *Bp = &S.bsdfs[prim_bsdf(S, h.prim)];
             DevBsdf Bl;
             if (Bp->textured) {
@@ -703,26 +743,27 @@ __global__ void __launch_bounds__(128, RT_VW_MINB_SAMPLE) k_vw_sample_surface(Re
 // MIS of what the ray found, throughput, Russian roulette
 // (VolPathTracing.cpp:300-367).  ro, rd: the sampled ray; h, seg, was,
 // flags: what evalTransmittanceFromSampledBSDF reported; L: the radiance with
-// this vertex's light-sample MIS.  Returns whether the path goes on (to the
+// this vertex's light-sample MIS; h1, was1, seg1: the first segment's hit and
+// its origin, kept for the next pass as its trace.  Returns whether the path goes on (to the
 // next round's trace queue, with its sampled ray).
+template <bool SCAT>
 __device__ __forceinline__ bool vw_finish_one(const RenderParams &P, const DevScene &S, int slot, int flags, Pcg32 rng,
-                                              float4 ro, float4 rd,
-                                              float4 seg, const Hit &h, bool was, C3 tr, C3 L, int depth,
-                                              float4 tpv, float4 bsv)
+                                              float4 ro, float4 rd, float4 seg, const Hit &h, bool was, const Hit &h1,
+                                              bool was1, float4 seg1, C3 tr, C3 L, int depth, float4 tpv, float4 bsv)
 {
     C3 T = rgb(tpv);
     float eta = tpv.w;
     const V3 d = xyz(rd);
     const int medium = __float_as_int(seg.w);
     bool done = false;
-    if (flags & VF_SCAT) {
+    if (SCAT) {
         T = T * rgb(bsv);
         if (was) {
             int hl = prim_light(S, h.prim);
             if (hl >= 0) {
-                Frame fr = vp_frame(S, h, xyz(seg), d);
+                Frame fr = hit_frame(S, h, xyz(seg), d);
                 C3 Le = area_le(S, hl, -d, fr.n);
-                float pl = vp_light_pdf(S, hl, fr.p, xyz(P.W.v_li1[slot]), xyz(P.W.v_li2[slot]),
+                float pl = light_pdf(S, hl, fr.p, xyz(P.W.v_li1[slot]), xyz(P.W.v_li2[slot]),
                                         xyz(P.W.v_li0[slot]));
                 float w = power_heuristic(bsv.w, pl);
                 L = L + ((T * Le) * tr) * w;
@@ -739,7 +780,7 @@ __device__ __forceinline__ bool vw_finish_one(const RenderParams &P, const DevSc
             int nl = prim_light(S, h.prim);
             if (nl >= 0) {
                 caught = nl;
-                fr = vp_frame(S, h, xyz(seg), d);
+                fr = hit_frame(S, h, xyz(seg), d);
                 Le = area_le(S, nl, -d, fr.n);
             }
         } else if (!(flags & VF_NEWM)) {
@@ -747,7 +788,7 @@ __device__ __forceinline__ bool vw_finish_one(const RenderParams &P, const DevSc
             if (S.env_light >= 0) { caught = S.env_light; isenv = true; Le = env_le(S.lights[S.env_light], d); }
         }
         if (caught >= 0) {
-            float pl = (flags & VF_DELTA) ? 0.f : vp_light_pdf(S, caught, xyz(P.W.v_p[slot]), fr.p, fr.n, d);
+            float pl = (flags & VF_DELTA) ? 0.f : light_pdf(S, caught, xyz(P.W.v_p[slot]), fr.p, fr.n, d);
             float w = power_heuristic(bsv.w, pl);
             L = L + (((T * Le) * f) * tr) * w;
             if (isenv && medium < 0) done = true;
@@ -768,9 +809,9 @@ __device__ __forceinline__ bool vw_finish_one(const RenderParams &P, const DevSc
         P.W.rng[slot] = rng;
         P.W.ray_o[slot] = ro;
         P.W.ray_d[slot] = rd;
-        P.W.hit[slot] = make_float4(h.t, h.u, h.v, __int_as_float(h.prim));
-        P.W.v_seg[slot] = seg;
-        P.W.flags[slot] = flags;
+        P.W.hit[slot] = make_float4(h1.t, h1.u, h1.v, __int_as_float(h1.prim));
+        P.W.v_seg[slot] = seg1;
+        P.W.flags[slot] = (flags & ~VF_WAS) | (was1 ? VF_WAS : 0);
         P.W.rad[slot] = f4c(L, __int_as_float(depth));
         P.W.tp[slot] = f4c(T, eta);
     }
@@ -801,14 +842,16 @@ __global__ void __launch_bounds__(128, RT_VW_MINB_TRSAMP) k_vw_trsamp_finish(Ren
         Hit h; h.t = hv.x; h.u = hv.y; h.v = hv.z; h.prim = __float_as_int(hv.w);
         float4 seg = P.W.v_seg[slot];
         V3 so = xyz(seg);
-        bool was;
+        Hit h1;
+        bool was, was1;
         int newm = -1;
         const C3 tr = vw_tr_sampled(S, make_ray(xyz(ro), xyz(rd), ro.w, rd.w), rng, __float_as_int(seg.w), h, so,
-                                    was, newm, limit);
-        flags = (flags & ~(VF_WAS | VF_NEWM)) | (was ? VF_WAS : 0) | (newm >= 0 ? VF_NEWM : 0);
+                                    was, h1, was1, newm, limit);
+        flags = (flags & ~VF_NEWM) | (newm >= 0 ? VF_NEWM : 0);
+        const float4 seg1 = was1 ? make_float4(ro.x, ro.y, ro.z, seg.w) : seg;
         seg = make_float4(so.x, so.y, so.z, seg.w);
         const float4 radv = P.W.rad[slot];
-        want = vw_finish_one(P, S, slot, flags, rng, ro, rd, seg, h, was, tr, rgb(radv), __float_as_int(radv.w),
+        want = vw_finish_one<false>(P, S, slot, flags, rng, ro, rd, seg, h, was, h1, was1, seg1, tr, rgb(radv), __float_as_int(radv.w),
                              P.W.tp[slot], P.W.bs[slot])
                    ? 1u
                    : 0u;
@@ -851,10 +894,12 @@ __global__ void __launch_bounds__(128, RT_VW_MINB_TRSAMP) k_vw_scatter(RenderPar
         const float4 hv = P.W.hit[slot];
         Hit h; h.t = hv.x; h.u = hv.y; h.v = hv.z; h.prim = __float_as_int(hv.w);
         V3 so = xyz(seg);
-        bool was;
+        Hit h1;
+        bool was, was1;
         int newm = -1;
-        const C3 tr = vw_tr_sampled(S, make_ray(xyz(ro), wo, 0.f, rd.w), rng, medium, h, so, was, newm, limit);
-        flags = (flags & ~(VF_WAS | VF_NEWM)) | (was ? VF_WAS : 0) | (newm >= 0 ? VF_NEWM : 0);
+        const C3 tr = vw_tr_sampled(S, make_ray(xyz(ro), wo, 0.f, rd.w), rng, medium, h, so, was, h1, was1, newm, limit);
+        flags = (flags & ~VF_NEWM) | (newm >= 0 ? VF_NEWM : 0);
+        const float4 seg1 = was1 ? make_float4(ro.x, ro.y, ro.z, seg.w) : seg;
         seg = make_float4(so.x, so.y, so.z, seg.w);
         // the light sample's MIS at the scatter point
         const float4 radv = P.W.rad[slot], tpv = P.W.tp[slot];
@@ -872,8 +917,8 @@ __global__ void __launch_bounds__(128, RT_VW_MINB_TRSAMP) k_vw_scatter(RenderPar
                 L = L + ((rgb(tpv) * value) * ev) * w;
             }
         }
-        want = vw_finish_one(P, S, slot, flags, rng, ro, rd, seg, h, was, tr, L, __float_as_int(radv.w), tpv,
-                             f4c(cfill(pfw), pfpdf))
+        want = vw_finish_one<true>(P, S, slot, flags, rng, ro, rd, seg, h, was, h1, was1, seg1, tr, L,
+                             __float_as_int(radv.w), tpv, f4c(cfill(pfw), pfpdf))
                    ? 1u
                    : 0u;
         }
