@@ -154,6 +154,12 @@ struct RenderParams {
     // rt_render_paths: slot i renders (pixel path_list[i].x, absolute sample
     // index path_list[i].y) and is not reduced into a film; null otherwise
     const int2 *path_list;
+    // rounds with at most this many paths are run to their end by one kernel
+    // (k_pt_tail, k_vw_tail); -1: none are
+    int tail_paths;
+    // host memory the tail kernels report to: entry round & 7 gets the paths
+    // the round leaves to the wavefront (0: all are done); null: no report
+    int *tail_host;
 };
 
 __device__ __forceinline__ int cur_round(const RenderParams &P, int round)
@@ -1079,6 +1085,17 @@ __global__ void __launch_bounds__(128) k_pt_finish(RenderParams P, int round)
     }
 }
 
+// The BSDF functions of any type, out of line: kernels that dispatch at run
+// time (the mixed queue's, VolPath's surfaces) call them from several places,
+// and with a switch over every type inlined at each the code overflowed the
+// instruction cache.
+__device__ __noinline__ C3 any_bsdf_sample(const DevBsdf &b, BsdfRec &r, V2 u, uint64_t aux_key)
+{
+    return bsdf_sample(b, r, u, aux_key);
+}
+__device__ __noinline__ C3 any_bsdf_eval(const DevBsdf &b, V3 wi, V3 wo) { return bsdf_eval(b, wi, wo); }
+__device__ __noinline__ float any_bsdf_pdf(const DevBsdf &b, V3 wi, V3 wo) { return bsdf_pdf(b, wi, wo); }
+
 // The BSDF functions of one shading queue (bsdf_queue), with the TwoSides
 // mirroring of bsdf_eval/bsdf_pdf/bsdf_sample.  Queue RT_QUEUE_DELTA holds
 // the smooth BSDFs, whose eval and pdf are zero; RT_QUEUE_MIXED holds every
@@ -1086,7 +1103,7 @@ __global__ void __launch_bounds__(128) k_pt_finish(RenderParams P, int round)
 template <int BT>
 __device__ __forceinline__ C3 bsdf_eval_t(const DevBsdf &b, V3 wi, V3 wo)
 {
-    if (BT == RT_QUEUE_MIXED) return bsdf_eval(b, wi, wo);
+    if (BT == RT_QUEUE_MIXED) return any_bsdf_eval(b, wi, wo);
     if (BT == RT_QUEUE_DELTA) return cfill(0.f);
     if (b.two_sided && !(wi.z > 0.f)) { wi.z = -wi.z; wo.z = -wo.z; }
     if (BT == 0) return diffuse_eval(b.albedo, wi, wo);
@@ -1098,7 +1115,7 @@ __device__ __forceinline__ C3 bsdf_eval_t(const DevBsdf &b, V3 wi, V3 wo)
 template <int BT>
 __device__ __forceinline__ float bsdf_pdf_t(const DevBsdf &b, V3 wi, V3 wo)
 {
-    if (BT == RT_QUEUE_MIXED) return bsdf_pdf(b, wi, wo);
+    if (BT == RT_QUEUE_MIXED) return any_bsdf_pdf(b, wi, wo);
     if (BT == RT_QUEUE_DELTA) return 0.f;
     if (b.two_sided && !(wi.z > 0.f)) { wi.z = -wi.z; wo.z = -wo.z; }
     if (BT == 0) return diffuse_pdf(wi, wo);
@@ -1123,7 +1140,7 @@ __device__ __forceinline__ C3 bsdf_sample1_t(const DevBsdf &b, BsdfRec &r, V2 s,
 template <int BT>
 __device__ __forceinline__ C3 bsdf_sample_t(const DevBsdf &b, BsdfRec &r, V2 s, uint64_t aux_key)
 {
-    if (BT == RT_QUEUE_MIXED) return bsdf_sample(b, r, s, aux_key);
+    if (BT == RT_QUEUE_MIXED) return any_bsdf_sample(b, r, s, aux_key);
     if (b.two_sided && !(r.wi.z > 0.f)) {
         r.wi.z = -r.wi.z;
         C3 res = bsdf_sample1_t<BT>(b, r, s, aux_key);
@@ -1188,14 +1205,16 @@ __device__ __forceinline__ void pt_shade_path(const RenderParams &P, const DevSc
     float4 hv = P.W.hit[slot];
     Hit h; h.t = hv.x; h.u = hv.y; h.v = hv.z; h.prim = __float_as_int(hv.w);
     Frame fr = hit_frame(S, h, o, d);
-    // the mixed queue's BSDF is a copy with its textures applied at
-    // the hit; the sorted queues read the scene's (untextured) BSDF
+    // a textured BSDF (mixed queue only) is a copy with its textures applied
+    // at the hit
+    const DevBsdf *Bp = &S.bsdfs[prim_bsdf(S, h.prim)];
     DevBsdf Bl;
-    if (BT == RT_QUEUE_MIXED) {
-        Bl = S.bsdfs[prim_bsdf(S, h.prim)];
-        if (Bl.textured) tex_apply(S, Bl, hit_uv(S, h, o, d));
+    if (BT == RT_QUEUE_MIXED && Bp->textured) {
+        Bl = *Bp;
+        tex_apply(S, Bl, hit_uv(S, h, o, d));
+        Bp = &Bl;
     }
-    const DevBsdf &B = BT == RT_QUEUE_MIXED ? Bl : S.bsdfs[prim_bsdf(S, h.prim)];
+    const DevBsdf &B = *Bp;
     bool done = false;
     // finish the previous vertex (its light sample and the emission
     // its BSDF-sampled ray found), update throughput, roulette
@@ -1326,6 +1345,113 @@ __global__ void __launch_bounds__(128, RT_SHADE_MINB) k_pt_shade(RenderParams P,
         }
         q_push(out_q, out_n, slot, (push_closest ? 1u : 0u) | (push_shadow ? 2u : 0u) | (push_end ? 4u : 0u));
     }
+}
+
+// ---------------------------------------------------------------- few paths
+// The start of a tail kernel on a round of n paths: true when they are few
+// enough to be run to their end here, false when the wavefront goes on (or
+// nothing is left).  What is left to the wavefront is reported to the host.
+__device__ __forceinline__ bool tail_begin(const RenderParams &P, RoundCounters *C, int n)
+{
+    const bool few = n > 0 && n <= P.tail_paths;
+    if (P.tail_host && blockIdx.x == 0 && threadIdx.x == 0) {
+        const int round = (int)(C - P.W.cnt);
+        *(volatile int *)(P.tail_host + (round & 7)) = few ? 0 : n;
+    }
+    return few;
+}
+// A thread's entries of the queue: [first, end) in steps of 32.  Each warp
+// takes a run of entries of the same length, as short as the grid allows, so
+// that a few paths do not share warps (and wait for one another's branches).
+__device__ __forceinline__ void tail_share(int n, int &first, int &end)
+{
+    const int warps = (gridDim.x * blockDim.x) >> 5, warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int run = (n + warps - 1) / warps;
+    first = warp * run + (threadIdx.x & 31);
+    end = imin(n, (warp + 1) * run);
+}
+// The end of a tail kernel that ran its round's paths: the last block empties
+// the round's queues, so that the kernels launched after it find nothing.
+// (Every block has read the counts before it adds itself here.)
+__device__ __forceinline__ void tail_end(RoundCounters *C)
+{
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    __threadfence();
+    if (atomicAdd(&C->tail_blocks, 1) == (int)gridDim.x - 1) {
+        C->closest = 0;
+        C->shadow = 0;
+        C->end = 0;
+    }
+}
+
+// Every path of the round (its closest-hit queue and the paths that ended
+// with a light sample pending) run to its end by one thread: trace, shade and
+// finish one after another, with the path's state in memory between them as
+// the wavefront keeps it.  Taken for a round with at most P.tail_paths paths.
+// A wavefront round is 4 to 10 launches, each of which waits for its slowest
+// path, whatever their number; here the rounds that are left cost one launch
+// together.  The films are the wavefront's: the same functions run on the
+// same state, over the binary tree, whose two traversals meet their leaves in
+// the same order.  A 33-path rt_render_paths call 0.52 -> 0.11 ms, a 171x121 x
+// 4 spp preview with refit 1.79 -> 0.94 ms, Cornell 256^2 x 16 spp (its last
+// rounds) 1.44 -> 1.32 ms.  Bound by the latency of one path's chain of loads;
+// two blocks per SM hold RT_PT_TAIL paths (3 to 8 blocks were 0-4 % slower).
+#ifndef RT_PT_TAIL_MINB
+#define RT_PT_TAIL_MINB 2
+#endif
+template <bool MULTI, bool ALL>
+__global__ void __launch_bounds__(128, RT_PT_TAIL_MINB) k_pt_tail(RenderParams P, int round)
+{
+    round = cur_round(P, round);
+    RoundCounters *C = &P.W.cnt[round];
+    const int nc = C->closest, n = nc + C->end;
+    if (!tail_begin(P, C, n)) return;
+    int first, end, n_closest = 0, n_shadow = 0;
+    tail_share(n, first, end);
+    for (int i = first; i < end; i += 32) {
+        const int slot = i < nc ? P.W.q_closest[i] : P.W.q_end[i - nc];
+        const DevScene &S = MULTI ? P.scenes[P.W.sid[slot]] : P.S;
+        for (;;) {
+            const int flags = P.W.flags[slot];
+            Hit h;
+            if (flags & F_NEE) {
+                const float4 o = P.W.sh_o[slot], d = P.W.sh_d[slot];
+                P.W.occl[slot] = trace_ray<true>(S, xyz(o), xyz(d), o.w, d.w, h) ? 1 : 0;
+                n_shadow++;
+            }
+            bool finish = (flags & F_END) != 0;
+            if (!finish) {
+                const float4 o = P.W.ray_o[slot], d = P.W.ray_d[slot];
+                h.t = d.w; h.u = h.v = 0.f;
+                trace_ray<false>(S, xyz(o), xyz(d), o.w, d.w, h);
+                P.W.hit[slot] = make_float4(h.t, h.u, h.v, __int_as_float(h.prim));
+                n_closest++;
+                finish = h.prim == -1 || prim_type(S, h.prim) < 0;
+            }
+            if (finish) {
+                pt_finish_path(P, S, slot);
+                break;
+            }
+            bool push_end = false, push_closest = false, push_shadow = false;
+            pt_shade_path<RT_QUEUE_MIXED, ALL>(P, S, slot, push_end, push_closest, push_shadow);
+            if (!push_closest && !push_end) break;
+        }
+    }
+    n_closest = __reduce_add_sync(0xffffffffu, n_closest);
+    n_shadow = __reduce_add_sync(0xffffffffu, n_shadow);
+    if ((threadIdx.x & 31) == 0) {
+        if (n_closest) atomicAdd(&P.stats[0], (unsigned long long)n_closest);
+        if (n_shadow) atomicAdd(&P.stats[1], (unsigned long long)n_shadow);
+    }
+    tail_end(C);
+}
+static void launch_pt_tail(const RenderParams &P, int r, int sm, cudaStream_t st)
+{
+    const int blocks = sm * RT_PT_TAIL_MINB;
+    if (P.scenes) k_pt_tail<true, false><<<blocks, 128, 0, st>>>(P, r);
+    else if (P.all_lights) k_pt_tail<false, true><<<blocks, 128, 0, st>>>(P, r);
+    else k_pt_tail<false, false><<<blocks, 128, 0, st>>>(P, r);
 }
 
 // The shading kernels of one round for the shading queues in `types` (bit
@@ -1788,6 +1914,10 @@ struct rt_ctx {
         cudaGraphExec_t exec;
     };
     std::vector<GraphEntry> gcache;
+    // what the tail kernels report (RenderParams::tail_host): page-locked host
+    // memory, its device address, and an event per round in flight
+    int *tail_host = nullptr, *tail_host_dev = nullptr;
+    cudaEvent_t tail_ev[2] = {nullptr, nullptr};
     int64_t graph_builds = 0, graph_hits = 0;
     // multi-scene batches (rt_internal_render_multi): scene table, work
     // items, concatenated tile orders and light CDFs (grown on demand)
@@ -1807,9 +1937,58 @@ static void graph_cache_clear(rt_ctx *c)
     c->gcache.clear();
 }
 
+// Rounds of at most this many paths end in the tail kernels.  Above the line
+// the wavefront's sorted, well-filled kernels are faster than one thread per
+// path.  PathTracingMIS, with 16k / 32k / 64k / 128k: Cornell 256^2 x 16 spp
+// 1.40 / 1.32 / 1.29 / 1.28 ms (1.44 without), the 83k-path preview 0.95 /
+// 0.95 / 1.01 / 1.50 ms.  VolPathTracing (longer paths, more divergence), with
+// 4k / 8k / 16k / 32k / 64k / 128k: grid medium 133x97 x 9 spp 1.81 / 1.78 /
+// 1.85 / 1.94 / 2.2 / 3.7 ms (3.24 without).
+#ifndef RT_PT_TAIL
+#define RT_PT_TAIL 32768
+#endif
+#ifndef RT_VW_TAIL
+#define RT_VW_TAIL 8192
+#endif
+// P.tail_paths and P.tail_host for a render over the tree of `width`.  The
+// tail kernels trace the binary tree, so renders over another tree (a tie may
+// name another triangle there) and counting renders (profiling level 2) have
+// none.
+static rt_status tail_setup(rt_ctx *c, int width, bool volpath, RenderParams &P)
+{
+    P.tail_paths = -1;
+    P.tail_host = nullptr;
+    if (c->profiling >= 2 || (!volpath && width != 2)) return RT_OK;
+    if (!c->tail_host) {
+        CK(cudaHostAlloc(&c->tail_host, 8 * sizeof(int), cudaHostAllocMapped));
+        CK(cudaHostGetDevicePointer(&c->tail_host_dev, c->tail_host, 0));
+        for (cudaEvent_t &e : c->tail_ev) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    }
+    P.tail_paths = volpath ? RT_VW_TAIL : RT_PT_TAIL;
+    P.tail_host = c->tail_host_dev;
+    return RT_OK;
+}
+// A round's tail kernel has been launched: mark it, so that tail_left can wait.
+static rt_status tail_mark(rt_ctx *c, const RenderParams &P, int r)
+{
+    if (P.tail_host) CK(cudaEventRecord(c->tail_ev[r & 1], c->stream));
+    return RT_OK;
+}
+// Paths round r left to the wavefront.  Called with the round's own kernels
+// already queued behind its tail kernel, so the device does not wait for the
+// host.
+static rt_status tail_left(rt_ctx *c, const RenderParams &P, int r, int &left)
+{
+    left = 1;
+    if (!P.tail_host) return RT_OK;
+    CK(cudaEventSynchronize(c->tail_ev[r & 1]));
+    left = *(volatile int *)(c->tail_host + (r & 7));
+    return RT_OK;
+}
+
 // kinds for per-kernel timing
 enum { K_CAMERA = 0, K_TRACE_C = 1, K_TRACE_A = 2, K_SHADE = 3, K_VOLPATH = 4, K_FILM = 5, K_RESOLVE = 6, K_SORT = 7,
-       K_KINDS = 8 };
+       K_TAIL = 8, K_KINDS = 9 };
 
 static void prof_begin(rt_ctx *c, int kind)
 {
@@ -2105,6 +2284,9 @@ rt_status rt_ctx_destroy(rt_ctx *c)
     cudaFree(c->stats);
     cudaFree(c->light_cdf);
     cudaFree(c->film);
+    if (c->tail_host) cudaFreeHost(c->tail_host);
+    for (cudaEvent_t e : c->tail_ev)
+        if (e) cudaEventDestroy(e);
     if (c->ev0) cudaEventDestroy(c->ev0);
     if (c->ev1) cudaEventDestroy(c->ev1);
     for (cudaEvent_t e : c->ev_pool) cudaEventDestroy(e);
@@ -3073,6 +3255,13 @@ static rt_status pt_batch_graph(rt_ctx *ctx, rt_scene *sc, const RenderParams &P
             if (bad(cudaMemsetAsync(P.round_dev, 0, sizeof(int), st), "memset")) break;
             k_camera<<<cam_blocks, 256, 0, st>>>(P);
             if (bad(cudaGetLastError(), "k_camera")) break;
+            const bool tail = P.tail_paths >= 0;
+            if (P.n_paths <= P.tail_paths) {
+                // few paths: no rounds
+                if (vw) k_vw_tail<<<sm * RT_VW_TAIL_MINB, 128, 0, st>>>(P, 0);
+                else launch_pt_tail(P, 0, sm, st);
+                if (bad(cudaGetLastError(), "tail kernel")) break;
+            } else {
             cudaStreamCaptureStatus cst;
             cudaGraph_t cg = nullptr;
             const cudaGraphNode_t *deps = nullptr;
@@ -3094,6 +3283,8 @@ static rt_status pt_batch_graph(rt_ctx *ctx, rt_scene *sc, const RenderParams &P
                     "body capture"))
                 break;
             body_capturing = true;
+            if (tail && vw) k_vw_tail<<<sm * RT_VW_TAIL_MINB, 128, 0, bs>>>(P, 0);
+            else if (tail) launch_pt_tail(P, 0, sm, bs);
             if (vw) {
                 // one VolPath round (the next round's trace queue is its
                 // counters' closest, which k_round_next tests)
@@ -3115,6 +3306,7 @@ static rt_status pt_batch_graph(rt_ctx *ctx, rt_scene *sc, const RenderParams &P
             if (bad(cudaStreamUpdateCaptureDependencies(st, &cn, nullptr, 1, cudaStreamSetCaptureDependencies),
                     "capture dependencies"))
                 break;
+            }
             if (box_film) k_film<<<(P.npix + 127) / 128, 128, 0, st>>>(P, film, Wd, accumulate);
             else k_film_wide<<<(int)((npix_all + 127) / 128), 128, 0, st>>>(P, film, t0, t1, tiles_x, bx, by);
             if (bad(cudaGetLastError(), "film kernel")) break;
@@ -3256,6 +3448,7 @@ rt_status rt_render(rt_ctx *ctx, rt_scene *sc, const rt_render_desc *rd, float *
     P.spp = rd->spp;
     P.sample_begin = rd->sample_begin;
     P.sort_threshold = ctx->sort_threshold;
+    P.tail_paths = -1;
     P.all_lights = rd->integrator == RT_INTEGRATOR_PATH_MIS && rd->strategy == RT_STRATEGY_ALL_LIGHTS;
     // shading queues in use: the scene's (textured BSDFs in the mixed one),
     // and the mixed one for bounces below the sort threshold
@@ -3266,13 +3459,17 @@ rt_status rt_render(rt_ctx *ctx, rt_scene *sc, const rt_render_desc *rd, float *
     // one CUDA graph per PathTracingMIS or VolPath-wavefront batch (rt_ctx_set_graphs)
     const bool use_graph = ctx->graphs && !ctx->profiling && !ctx->ray_sort &&
                            (rd->integrator == RT_INTEGRATOR_PATH_MIS || vw);
-    int graph_batches = 0;
+    int graph_batches = 0, few_batches = 0;
     if (use_graph) {
         if (!ctx->round_dev) CK(cudaMalloc(&ctx->round_dev, sizeof(int)));
         if (!ctx->body_stream) CK(cudaStreamCreateWithFlags(&ctx->body_stream, cudaStreamNonBlocking));
         if (!ctx->cap_stream) CK(cudaStreamCreateWithFlags(&ctx->cap_stream, cudaStreamNonBlocking));
         P.round_dev = ctx->round_dev;
     }
+    const int width = trace_width(ctx, sc);
+    if ((rd->integrator == RT_INTEGRATOR_PATH_MIS || vw) && (s = tail_setup(ctx, width, vw, P)) != RT_OK) return s;
+    if (use_graph) P.tail_host = nullptr;   // the graph's loop tests the counters itself
+    const bool tail = P.tail_paths >= 0;
     ctx->ev_used = 0;
     CK(cudaEventRecord(ctx->ev0, st));
     for (int t0 = 0; t0 < ntiles; t0 += tiles_per_batch) {
@@ -3286,6 +3483,7 @@ rt_status rt_render(rt_ctx *ctx, rt_scene *sc, const rt_render_desc *rd, float *
                                     round_buf, vw)) != RT_OK)
                 return s;
             graph_batches++;
+            few_batches += P.n_paths <= P.tail_paths;
             continue;
         }
         CK(cudaMemsetAsync(ctx->W.pix_irregular, 0, (size_t)P.npix, st));
@@ -3300,6 +3498,12 @@ rt_status rt_render(rt_ctx *ctx, rt_scene *sc, const rt_render_desc *rd, float *
             // one round = one vol_step of every live path (five kernels)
             prof_begin(ctx, K_VOLPATH);
             for (int r = 0; r < max_rounds; r++) {
+                if (tail && r > 0) {
+                    k_vw_tail<<<sm * RT_VW_TAIL_MINB, 128, 0, st>>>(P, r);
+                    launches++;
+                    if ((s = launch_check("k_vw_tail")) != RT_OK || (s = tail_mark(ctx, P, r)) != RT_OK) return s;
+                    if (P.n_paths <= P.tail_paths) break;
+                }
                 k_vw_trace_step<<<sm * RT_VW_MINB_STEP, 128, 0, st>>>(P, r);
                 k_vw_shadow<<<sm * RT_VW_MINB_SHADOW, 128, 0, st>>>(P, r);
                 k_vw_scatter<<<sm * RT_VW_MINB_TRSAMP, 128, 0, st>>>(P, r);
@@ -3307,6 +3511,12 @@ rt_status rt_render(rt_ctx *ctx, rt_scene *sc, const rt_render_desc *rd, float *
                 k_vw_trsamp_finish<<<sm * RT_VW_MINB_TRSAMP, 128, 0, st>>>(P, r);
                 launches += 5;
                 if ((s = launch_check("VolPath round")) != RT_OK) return s;
+                if (tail) {
+                    int left = 1;
+                    if (r > 0 && (s = tail_left(ctx, P, r, left)) != RT_OK) return s;
+                    if (left == 0) break;
+                    continue;
+                }
                 if ((r & 3) == 3 && r + 1 < max_rounds) {
                     int nq = 0;
                     CK(cudaMemcpyAsync(&nq, &ctx->W.cnt[r + 1].closest, sizeof(int), cudaMemcpyDeviceToHost, st));
@@ -3328,7 +3538,14 @@ rt_status rt_render(rt_ctx *ctx, rt_scene *sc, const rt_render_desc *rd, float *
             for (int r = 0; r < max_rounds; r++) {
                 int ri = r;
                 const bool cnt2 = ctx->profiling >= 2;
-                const int width = trace_width(ctx, sc);
+                if (tail && (r > 0 || P.n_paths <= P.tail_paths)) {
+                    prof_begin(ctx, K_TAIL);
+                    launch_pt_tail(P, r, sm, st);
+                    prof_end(ctx);
+                    launches++;
+                    if ((s = launch_check("k_pt_tail")) != RT_OK || (s = tail_mark(ctx, P, r)) != RT_OK) return s;
+                    if (r == 0) break;
+                }
                 if (ctx->ray_sort && ri > 0) {
                     prof_begin(ctx, K_SORT);
                     if ((s = sort_rays(ctx, P, ri, 0, launches)) != RT_OK) return s;
@@ -3351,6 +3568,12 @@ rt_status rt_render(rt_ctx *ctx, rt_scene *sc, const rt_render_desc *rd, float *
                 trace_c_launches++;
                 trace_a_launches++;
                 if ((s = launch_check("pt round")) != RT_OK) return s;
+                if (tail) {
+                    int left = 1;
+                    if (r > 0 && (s = tail_left(ctx, P, r, left)) != RT_OK) return s;
+                    if (left == 0) break;
+                    continue;
+                }
                 // cheap early exit: peek at the survivor counts every 4 rounds
                 if ((r & 3) == 3 && r + 1 < max_rounds) {
                     RoundCounters nc;
@@ -3383,7 +3606,7 @@ rt_status rt_render(rt_ctx *ctx, rt_scene *sc, const rt_render_desc *rd, float *
     cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1);
     std::memset(&ctx->last, 0, sizeof(ctx->last));
     ctx->last.kernel_ms = ms;
-    double kt[K_KINDS] = {0, 0, 0, 0, 0, 0, 0, 0};
+    double kt[K_KINDS] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
     for (size_t i = 0; i < ctx->ev_used; i++) {
         float e = 0.f;
         cudaEventElapsedTime(&e, ctx->ev_pool[2 * i], ctx->ev_pool[2 * i + 1]);
@@ -3392,7 +3615,7 @@ rt_status rt_render(rt_ctx *ctx, rt_scene *sc, const rt_render_desc *rd, float *
     ctx->last.camera_ms = kt[K_CAMERA];
     ctx->last.trace_closest_ms = kt[K_TRACE_C];
     ctx->last.trace_any_ms = kt[K_TRACE_A];
-    ctx->last.shade_ms = kt[K_SHADE] + kt[K_RESOLVE];
+    ctx->last.shade_ms = kt[K_SHADE] + kt[K_RESOLVE] + kt[K_TAIL];
     ctx->last.resolve_ms = kt[K_RESOLVE];
     ctx->last.sort_ms = kt[K_SORT];
     ctx->last.volpath_ms = kt[K_VOLPATH];
@@ -3410,8 +3633,9 @@ rt_status rt_render(rt_ctx *ctx, rt_scene *sc, const rt_render_desc *rd, float *
     if (graph_batches) {
         // camera and film per batch, the rounds' kernels and k_round_next
         const int64_t rounds = (int64_t)stats[7];
-        const int per_round = vw ? 5 + 1 : 3 + __builtin_popcount(types) + 1;
-        launches += 2 * (int64_t)graph_batches + rounds * per_round;
+        // (a graph of few paths: the tail kernel instead of rounds)
+        const int per_round = (vw ? 5 : 3 + __builtin_popcount(types)) + 1 + (tail ? 1 : 0);
+        launches += 2 * (int64_t)graph_batches + rounds * per_round + few_batches;
         trace_c_launches += rounds;
         trace_a_launches += rounds;
     }
@@ -3604,6 +3828,8 @@ rt_status rt_internal_render_multi(rt_ctx *ctx, rt_scene *const *scenes, const r
     P.sort_threshold = ctx->sort_threshold;
     P.scenes = ctx->m_scenes;
     P.items = ctx->m_items;
+    if ((s = tail_setup(ctx, 2, false, P)) != RT_OK) { release(); return s; }
+    const bool tail = P.tail_paths >= 0;
     const int sm = ctx->sm_count > 0 ? ctx->sm_count : 1;
     const int trace_blocks = sm * ctx->trace_bpsm, shade_blocks = sm * ctx->shade_bpsm;
     int64_t launches = 0, rounds_run = 0, total_paths = 0;
@@ -3624,6 +3850,14 @@ rt_status rt_internal_render_multi(rt_ctx *ctx, rt_scene *const *scenes, const r
         launches++;
         if ((s = launch_check("k_camera_multi")) != RT_OK) { release(); return s; }
         for (int r = 0; r < max_rounds; r++) {
+            if (tail && (r > 0 || P.n_paths <= P.tail_paths)) {
+                prof_begin(ctx, K_TAIL);
+                launch_pt_tail(P, r, sm, st);
+                prof_end(ctx);
+                launches++;
+                if ((s = launch_check("k_pt_tail")) != RT_OK || (s = tail_mark(ctx, P, r)) != RT_OK) { release(); return s; }
+                if (r == 0) break;
+            }
             prof_begin(ctx, K_TRACE_C);
             k_trace<false, false, true><<<trace_blocks, 128, 0, st>>>(P, r);
             prof_end(ctx);
@@ -3645,6 +3879,12 @@ rt_status rt_internal_render_multi(rt_ctx *ctx, rt_scene *const *scenes, const r
             launches += 3 + __builtin_popcount(types);
             rounds_run++;
             if ((s = launch_check("multi-scene round")) != RT_OK) { release(); return s; }
+            if (tail) {
+                int left = 1;
+                if (r > 0 && (s = tail_left(ctx, P, r, left)) != RT_OK) { release(); return s; }
+                if (left == 0) break;
+                continue;
+            }
             if ((r & 3) == 3 && r + 1 < max_rounds) {
                 RoundCounters nc;
                 CK(cudaMemcpyAsync(&nc, &ctx->W.cnt[r + 1], sizeof(nc), cudaMemcpyDeviceToHost, st));
@@ -3674,7 +3914,7 @@ rt_status rt_internal_render_multi(rt_ctx *ctx, rt_scene *const *scenes, const r
     cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1);
     std::memset(&ctx->last, 0, sizeof(ctx->last));
     ctx->last.kernel_ms = ms;
-    double kt[K_KINDS] = {0, 0, 0, 0, 0, 0, 0, 0};
+    double kt[K_KINDS] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
     for (size_t i = 0; i < ctx->ev_used; i++) {
         float e = 0.f;
         cudaEventElapsedTime(&e, ctx->ev_pool[2 * i], ctx->ev_pool[2 * i + 1]);
@@ -3683,7 +3923,7 @@ rt_status rt_internal_render_multi(rt_ctx *ctx, rt_scene *const *scenes, const r
     ctx->last.camera_ms = kt[K_CAMERA];
     ctx->last.trace_closest_ms = kt[K_TRACE_C];
     ctx->last.trace_any_ms = kt[K_TRACE_A];
-    ctx->last.shade_ms = kt[K_SHADE] + kt[K_RESOLVE];
+    ctx->last.shade_ms = kt[K_SHADE] + kt[K_RESOLVE] + kt[K_TAIL];
     ctx->last.resolve_ms = kt[K_RESOLVE];
     ctx->last.film_ms = kt[K_FILM];
     ctx->last.trace_closest_launches = rounds_run;
@@ -3760,10 +4000,22 @@ rt_status rt_render_paths(rt_ctx *ctx, rt_scene *sc, const rt_render_desc *rd, c
         P.path_list = (const int2 *)tmp;
         const int sm = ctx->sm_count > 0 ? ctx->sm_count : 1;
         rt_status e;
+        const int width = trace_width(ctx, sc);
+        P.tail_paths = -1;
+        if ((rd->integrator == RT_INTEGRATOR_PATH_MIS || vw) && (e = tail_setup(ctx, width, vw, P)) != RT_OK) return e;
+        P.tail_host = nullptr;
+        const bool tail = P.tail_paths >= 0, few = n <= P.tail_paths;
         k_camera<<<std::min((n + 255) / 256, sm * 16), 256, 0, st>>>(P);
         if ((e = launch_check("k_camera (paths)")) != RT_OK) return e;
-        if (vw) {
+        if (vw && few) {
+            k_vw_tail<<<sm * RT_VW_TAIL_MINB, 128, 0, st>>>(P, 0);
+            if ((e = launch_check("k_vw_tail (paths)")) != RT_OK) return e;
+        } else if (few) {
+            launch_pt_tail(P, 0, sm, st);
+            if ((e = launch_check("k_pt_tail (paths)")) != RT_OK) return e;
+        } else if (vw) {
             for (int r = 0; r < max_rounds; r++) {
+                if (tail && r > 0) k_vw_tail<<<sm * RT_VW_TAIL_MINB, 128, 0, st>>>(P, r);
                 k_vw_trace_step<<<sm * RT_VW_MINB_STEP, 128, 0, st>>>(P, r);
                 k_vw_shadow<<<sm * RT_VW_MINB_SHADOW, 128, 0, st>>>(P, r);
                 k_vw_scatter<<<sm * RT_VW_MINB_TRSAMP, 128, 0, st>>>(P, r);
@@ -3782,8 +4034,8 @@ rt_status rt_render_paths(rt_ctx *ctx, rt_scene *sc, const rt_render_desc *rd, c
         } else {
             const int types = sc->bsdf_types | (P.sort_threshold > 0 ? 1 << RT_QUEUE_MIXED : 0);
             const int tb = sm * ctx->trace_bpsm, sb = sm * ctx->shade_bpsm;
-            const int width = trace_width(ctx, sc);
             for (int r = 0; r < max_rounds; r++) {
+                if (tail && r > 0) launch_pt_tail(P, r, sm, st);
                 launch_trace(width, P, r, false, false, tb, st);
                 launch_trace(width, P, r, true, false, tb, st);
                 k_pt_finish<<<sb, 128, 0, st>>>(P, r);
@@ -4143,6 +4395,10 @@ extern "C" rt_status rt_render_tile_static(rt_ctx *ctx, rt_scene *sc, const rt_r
     if (rd->integrator == RT_INTEGRATOR_VOLPATH) {
         k_volpath<<<sm * RT_VOLPATH_GRID, 128, 0, st>>>(Pm, work);
         if ((s = launch_check("k_volpath")) != RT_OK) return s;
+    } else if (trace_width(ctx, sc) == 2 && paths <= RT_PT_TAIL) {
+        Pm.tail_paths = RT_PT_TAIL;
+        launch_pt_tail(Pm, 0, sm, st);
+        if ((s = launch_check("k_pt_tail (static)")) != RT_OK) return s;
     } else {
         const int blocks = sm * 8;
         for (int r = 0; r < rounds; r++) {

@@ -20,7 +20,8 @@ struct RoundCounters {   // one per wavefront round, zeroed per batch
     int closest, shadow, wc_closest, wc_shadow;
     int mat[RT_NQUEUE];  // paths per shading queue (material-sorted), in the mixed queue, to finish
     int end;             // paths that ended in shading with a light sample pending
-    int pad[3];
+    int tail_blocks;     // blocks of the round's tail kernel that have finished
+    int pad[2];
 };
 
 struct Wave {

@@ -31,12 +31,6 @@ __device__ __noinline__ bool vp_medium_sample(const DevMedium &m, Ray r, Pcg32 &
 {
     return medium_sample(m, r, rng, t, w, em, limit);
 }
-__device__ __noinline__ C3 vp_bsdf_sample(const DevBsdf &b, BsdfRec &r, V2 u, uint64_t aux_key)
-{
-    return bsdf_sample(b, r, u, aux_key);
-}
-__device__ __noinline__ C3 vp_bsdf_eval(const DevBsdf &b, V3 wi, V3 wo) { return bsdf_eval(b, wi, wo); }
-__device__ __noinline__ float vp_bsdf_pdf(const DevBsdf &b, V3 wi, V3 wo) { return bsdf_pdf(b, wi, wo); }
 __device__ __noinline__ void vp_light_sample(const DevScene &S, int idx, V3 p, V2 u, LightRec &li)
 {
     light_sample(S, idx, p, u, li);
@@ -234,15 +228,15 @@ __device__ bool vol_step(const DevScene &S, VolState &st, Pcg32 &rng, int max_de
         if (!iszero(value)) {
             V3 wi = to_local(fr, li.to_light), wo = to_local(fr, -ray.d);
             float ct = fabsf(wi.z);
-            float bp = li.delta ? 0.f : vp_bsdf_pdf(B, wi, wo);   // VolPathTracing.cpp:222
+            float bp = li.delta ? 0.f : any_bsdf_pdf(B, wi, wo);   // VolPathTracing.cpp:222
             float w = power_heuristic(li.pdf, bp);
-            L = L + (((T * value) * vp_bsdf_eval(B, wi, wo)) * ct) * w;
+            L = L + (((T * value) * any_bsdf_eval(B, wi, wo)) * ct) * w;
         }
         BsdfRec r;
         r.wi = to_local(fr, -ray.d); r.wo = v3(0, 0, 0);
         r.type = BT_ALL; r.rel_eta = 1.f; r.pdf = -1.f;
         V2 bu = next2d(rng);
-        C3 f = vp_bsdf_sample(B, r, bu, rng.state);
+        C3 f = any_bsdf_sample(B, r, bu, rng.state);
         if (iszero(f)) return false;
         V3 pfrom = fr.p;
         ray = make_ray(fr.p, to_world(fr, r.wo), RT_EPSILON, RT_MAX_REAL);
@@ -475,6 +469,9 @@ __device__ __forceinline__ C3 vw_transmittance(const DevScene &S, Ray ray, int m
 #ifndef RT_VW_MINB_TRSAMP
 #define RT_VW_MINB_TRSAMP RT_VW_MINB
 #endif
+// Each kernel's work on one path is a function of its own (vw_*_path), which
+// returns the queues the path goes to (bits, in the order of the kernel's
+// queue list); k_vw_tail calls them one after another.
 // whole warps run every pass of the loop (VW_LIVE: the lane has a path), so
 // that the pushes at its end are the warp's
 #define VW_LOOP(COUNT, QUEUE)                                                                      \
@@ -503,6 +500,116 @@ __device__ __forceinline__ int *vw_trace_queue(const RenderParams &P, int round)
 // takes its hit from there (vw_finish_one stores it); only camera rays and
 // the rays behind a null boundary are traced here.  They come first in the
 // queue, so few warps mix the two.  128^3 grid-medium frame: 64.4 -> 63.6 ms.
+__device__ __forceinline__ unsigned vw_step_path(const RenderParams &P, const DevScene &S, int slot, int &limit)
+{
+    unsigned want = 0;
+    // ---- the trace (k_vw_trace)
+    int flags = P.W.flags[slot];
+    const float4 ro = P.W.ray_o[slot], rd = P.W.ray_d[slot];
+    float4 radv = P.W.rad[slot];
+    float4 seg;
+    Hit h;
+    const bool traces = (flags & (VF_FIRST | VF_NULLX)) != 0;
+    if (flags & VF_FIRST) {
+        h.t = RT_MAX_REAL; h.u = h.v = 0.f; h.prim = -1;
+        seg = make_float4(0.f, 0.f, 0.f, __int_as_float(S.cam.medium));
+        flags = VF_EMISSION;
+    } else {
+        const float4 hv = P.W.hit[slot];
+        h.t = hv.x; h.u = hv.y; h.v = hv.z; h.prim = __float_as_int(hv.w);
+        seg = P.W.v_seg[slot];
+        if (!(flags & VF_NULLX)) {   // the trace that ends a bounce
+            flags &= ~VF_EMISSION;
+            radv.w = __int_as_float(__float_as_int(radv.w) + 1);
+        }
+    }
+    if (traces) {
+        Hit nh;
+        const bool was = trace_ray<false>(S, xyz(ro), xyz(rd), ro.w, rd.w, nh);
+        if (was) {
+            h = nh;
+            seg = make_float4(ro.x, ro.y, ro.z, seg.w);
+        }
+        flags = (flags & ~(VF_NULLX | VF_WAS)) | (was ? VF_WAS : 0);
+        P.W.hit[slot] = make_float4(h.t, h.u, h.v, __int_as_float(h.prim));
+    }
+    // ---- the step (k_vw_step)
+    const float4 tpv = P.W.tp[slot];
+    C3 L = rgb(radv), T = rgb(tpv);
+    const int depth = __float_as_int(radv.w);
+    bool push_shadow = false, push_sample = false, push_trace = false;
+    int guard = (flags >> VF_GUARD_SHIFT) + 1;
+    if (depth >= P.max_depth) {
+        vw_done(P, slot, L);
+    } else if (guard > (1 << 16)) {
+        limit = 1;
+        vw_done(P, slot, L);
+    } else {
+        Pcg32 rng = P.W.rng[slot];
+        Ray ray = make_ray(xyz(ro), xyz(rd), ro.w, rd.w);
+        int medium = __float_as_int(seg.w);
+        float t = 0.f;
+        C3 wm = cfill(0.f), em = cfill(0.f);
+        bool scattered = false;
+        if (medium >= 0)
+            scattered = medium_sample(S.media[medium], make_ray(ray.o, ray.d, ray.mint, h.t), rng, t, wm, em, limit);
+        bool done = false, vertex = false;
+        V3 vp = v3(0.f, 0.f, 0.f);
+        if (scattered) {
+            L = L + T * em;
+            T = T * wm;
+            vp = ray.o + t * ray.d;
+            flags |= VF_SCAT;
+            vertex = true;
+        } else {
+            flags &= ~VF_SCAT;
+            if (medium >= 0) {
+                L = L + T * em;
+                T = T * wm;
+            }
+            if (!(flags & VF_WAS)) {
+                if ((flags & VF_EMISSION) && S.env_light >= 0) L = L + T * env_le(S.lights[S.env_light], ray.d);
+                done = true;
+            } else {
+                Frame fr = hit_frame(S, h, xyz(seg), ray.d);
+                if (prim_bsdf(S, h.prim) < 0) {
+                    // null boundary: through, without a bounce
+                    ray = make_ray(fr.p, ray.d, RT_EPSILON, RT_MAX_REAL);
+                    if (prim_interior(S, h.prim) != prim_exterior(S, h.prim))
+                        medium = dot(fr.n, ray.d) < 0.f ? prim_interior(S, h.prim) : prim_exterior(S, h.prim);
+                    P.W.ray_o[slot] = f4(ray.o, ray.mint);
+                    P.W.ray_d[slot] = f4(ray.d, ray.maxt);
+                    flags |= VF_NULLX;
+                    push_trace = true;
+                } else {
+                    int hl = prim_light(S, h.prim);
+                    if ((flags & VF_EMISSION) && hl >= 0) L = L + T * area_le(S, hl, -ray.d, fr.n);
+                    vp = fr.p;
+                    vertex = true;
+                }
+            }
+        }
+        if (vertex) {
+            LightRec li;
+            float lw;
+            push_shadow = vw_light_pick(S, vp, rng, li, lw);
+            push_sample = !push_shadow;
+            vw_store_light(P, slot, li, vp, lw);
+            flags &= ~VF_HASVAL;
+        }
+        if (done) {
+            vw_done(P, slot, L);
+        } else {
+            P.W.rng[slot] = rng;
+            P.W.rad[slot] = f4c(L, __int_as_float(depth));
+            P.W.tp[slot] = f4c(T, tpv.w);
+            P.W.v_seg[slot] = make_float4(seg.x, seg.y, seg.z, __int_as_float(medium));
+            P.W.flags[slot] = (flags & ((1 << VF_GUARD_SHIFT) - 1)) | (guard << VF_GUARD_SHIFT);
+        }
+    }
+    want = push_shadow ? 1u : push_sample ? ((flags & VF_SCAT) ? 2u : 4u) : push_trace ? 8u : 0u;
+    return want;
+}
 __global__ void __launch_bounds__(128, RT_VW_MINB_STEP) k_vw_trace_step(RenderParams P, int round)
 {
     round = cur_round(P, round);
@@ -516,119 +623,29 @@ __global__ void __launch_bounds__(128, RT_VW_MINB_STEP) k_vw_trace_step(RenderPa
     VW_LOOP(C->closest, vw_trace_queue(P, round))
     {
         const int slot = VW_LIVE ? qin_[i_] : 0;
-        unsigned want = 0;
-        if (VW_LIVE) {
-        // ---- the trace (k_vw_trace)
-        int flags = P.W.flags[slot];
-        const float4 ro = P.W.ray_o[slot], rd = P.W.ray_d[slot];
-        float4 radv = P.W.rad[slot];
-        float4 seg;
-        Hit h;
-        const bool traces = (flags & (VF_FIRST | VF_NULLX)) != 0;
-        if (flags & VF_FIRST) {
-            h.t = RT_MAX_REAL; h.u = h.v = 0.f; h.prim = -1;
-            seg = make_float4(0.f, 0.f, 0.f, __int_as_float(S.cam.medium));
-            flags = VF_EMISSION;
-        } else {
-            const float4 hv = P.W.hit[slot];
-            h.t = hv.x; h.u = hv.y; h.v = hv.z; h.prim = __float_as_int(hv.w);
-            seg = P.W.v_seg[slot];
-            if (!(flags & VF_NULLX)) {   // the trace that ends a bounce
-                flags &= ~VF_EMISSION;
-                radv.w = __int_as_float(__float_as_int(radv.w) + 1);
-            }
-        }
-        if (traces) {
-            Hit nh;
-            const bool was = trace_ray<false>(S, xyz(ro), xyz(rd), ro.w, rd.w, nh);
-            if (was) {
-                h = nh;
-                seg = make_float4(ro.x, ro.y, ro.z, seg.w);
-            }
-            flags = (flags & ~(VF_NULLX | VF_WAS)) | (was ? VF_WAS : 0);
-            P.W.hit[slot] = make_float4(h.t, h.u, h.v, __int_as_float(h.prim));
-        }
-        // ---- the step (k_vw_step)
-        const float4 tpv = P.W.tp[slot];
-        C3 L = rgb(radv), T = rgb(tpv);
-        const int depth = __float_as_int(radv.w);
-        bool push_shadow = false, push_sample = false, push_trace = false;
-        int guard = (flags >> VF_GUARD_SHIFT) + 1;
-        if (depth >= P.max_depth) {
-            vw_done(P, slot, L);
-        } else if (guard > (1 << 16)) {
-            limit = 1;
-            vw_done(P, slot, L);
-        } else {
-            Pcg32 rng = P.W.rng[slot];
-            Ray ray = make_ray(xyz(ro), xyz(rd), ro.w, rd.w);
-            int medium = __float_as_int(seg.w);
-            float t = 0.f;
-            C3 wm = cfill(0.f), em = cfill(0.f);
-            bool scattered = false;
-            if (medium >= 0)
-                scattered = medium_sample(S.media[medium], make_ray(ray.o, ray.d, ray.mint, h.t), rng, t, wm, em, limit);
-            bool done = false, vertex = false;
-            V3 vp = v3(0.f, 0.f, 0.f);
-            if (scattered) {
-                L = L + T * em;
-                T = T * wm;
-                vp = ray.o + t * ray.d;
-                flags |= VF_SCAT;
-                vertex = true;
-            } else {
-                flags &= ~VF_SCAT;
-                if (medium >= 0) {
-                    L = L + T * em;
-                    T = T * wm;
-                }
-                if (!(flags & VF_WAS)) {
-                    if ((flags & VF_EMISSION) && S.env_light >= 0) L = L + T * env_le(S.lights[S.env_light], ray.d);
-                    done = true;
-                } else {
-                    Frame fr = hit_frame(S, h, xyz(seg), ray.d);
-                    if (prim_bsdf(S, h.prim) < 0) {
-                        // null boundary: through, without a bounce
-                        ray = make_ray(fr.p, ray.d, RT_EPSILON, RT_MAX_REAL);
-                        if (prim_interior(S, h.prim) != prim_exterior(S, h.prim))
-                            medium = dot(fr.n, ray.d) < 0.f ? prim_interior(S, h.prim) : prim_exterior(S, h.prim);
-                        P.W.ray_o[slot] = f4(ray.o, ray.mint);
-                        P.W.ray_d[slot] = f4(ray.d, ray.maxt);
-                        flags |= VF_NULLX;
-                        push_trace = true;
-                    } else {
-                        int hl = prim_light(S, h.prim);
-                        if ((flags & VF_EMISSION) && hl >= 0) L = L + T * area_le(S, hl, -ray.d, fr.n);
-                        vp = fr.p;
-                        vertex = true;
-                    }
-                }
-            }
-            if (vertex) {
-                LightRec li;
-                float lw;
-                push_shadow = vw_light_pick(S, vp, rng, li, lw);
-                push_sample = !push_shadow;
-                vw_store_light(P, slot, li, vp, lw);
-                flags &= ~VF_HASVAL;
-            }
-            if (done) {
-                vw_done(P, slot, L);
-            } else {
-                P.W.rng[slot] = rng;
-                P.W.rad[slot] = f4c(L, __int_as_float(depth));
-                P.W.tp[slot] = f4c(T, tpv.w);
-                P.W.v_seg[slot] = make_float4(seg.x, seg.y, seg.z, __int_as_float(medium));
-                P.W.flags[slot] = (flags & ((1 << VF_GUARD_SHIFT) - 1)) | (guard << VF_GUARD_SHIFT);
-            }
-        }
-        want = push_shadow ? 1u : push_sample ? ((flags & VF_SCAT) ? 2u : 4u) : push_trace ? 8u : 0u;
-        }
+        const unsigned want = VW_LIVE ? vw_step_path(P, S, slot, limit) : 0u;
         q_push(out_q, out_n, slot, want);
     }
     if (limit) atomicOr(P.limit_flag, RT_LIM_VOLPATH);
 }
 
+__device__ __forceinline__ unsigned vw_shadow_path(const RenderParams &P, const DevScene &S, int slot, int &limit)
+{
+    unsigned want = 0;
+    Pcg32 rng = P.W.rng[slot];
+    float4 pv = P.W.v_p[slot], l0 = P.W.v_li0[slot], l1 = P.W.v_li1[slot], iv = P.W.v_val[slot];
+    const int medium = __float_as_int(P.W.v_seg[slot].w);
+    C3 tr = vw_transmittance(S, make_ray(xyz(pv), xyz(l0), RT_EPSILON, l0.w - RT_EPSILON), medium, rng, limit);
+    float pdf = l1.w * pv.w;
+    C3 value = (tr * rgb(iv)) / pdf;
+    P.W.v_li1[slot] = make_float4(l1.x, l1.y, l1.z, pdf);
+    P.W.v_val[slot] = f4c(value, 0.f);
+    P.W.rng[slot] = rng;
+    const int flags = P.W.flags[slot] | VF_HASVAL;
+    P.W.flags[slot] = flags;
+    want = (flags & VF_SCAT) ? 1u : 2u;
+    return want;
+}
 __global__ void __launch_bounds__(128, RT_VW_MINB_SHADOW) k_vw_shadow(RenderParams P, int round)
 {
     round = cur_round(P, round);
@@ -640,21 +657,7 @@ __global__ void __launch_bounds__(128, RT_VW_MINB_SHADOW) k_vw_shadow(RenderPara
     VW_LOOP(C->shadow, P.W.q_shadow)
     {
         const int slot = VW_LIVE ? qin_[i_] : 0;
-        unsigned want = 0;
-        if (VW_LIVE) {
-        Pcg32 rng = P.W.rng[slot];
-        float4 pv = P.W.v_p[slot], l0 = P.W.v_li0[slot], l1 = P.W.v_li1[slot], iv = P.W.v_val[slot];
-        const int medium = __float_as_int(P.W.v_seg[slot].w);
-        C3 tr = vw_transmittance(S, make_ray(xyz(pv), xyz(l0), RT_EPSILON, l0.w - RT_EPSILON), medium, rng, limit);
-        float pdf = l1.w * pv.w;
-        C3 value = (tr * rgb(iv)) / pdf;
-        P.W.v_li1[slot] = make_float4(l1.x, l1.y, l1.z, pdf);
-        P.W.v_val[slot] = f4c(value, 0.f);
-        P.W.rng[slot] = rng;
-        const int flags = P.W.flags[slot] | VF_HASVAL;
-        P.W.flags[slot] = flags;
-        want = (flags & VF_SCAT) ? 1u : 2u;
-        }
+        const unsigned want = VW_LIVE ? vw_shadow_path(P, S, slot, limit) : 0u;
         q_push(out_q, out_n, slot, want);
     }
     if (limit) atomicOr(P.limit_flag, RT_LIM_VOLPATH);
@@ -664,6 +667,69 @@ __global__ void __launch_bounds__(128, RT_VW_MINB_SHADOW) k_vw_shadow(RenderPara
 // mat[4]): the light sample's MIS with the BSDF (textures applied), the BSDF
 // sample and the new ray.  Scatter points in media (mat[1]) go through
 // k_vw_scatter, which continues into the sampled ray's transmittance.
+__device__ __forceinline__ unsigned vw_surface_path(const RenderParams &P, const DevScene &S, int slot)
+{
+    unsigned want = 0;
+    int flags = P.W.flags[slot];
+    Pcg32 rng = P.W.rng[slot];
+    float4 radv = P.W.rad[slot], tpv = P.W.tp[slot];
+    C3 L = rgb(radv), T = rgb(tpv);
+    float4 ro = P.W.ray_o[slot], rd = P.W.ray_d[slot];
+    Ray ray = make_ray(xyz(ro), xyz(rd), ro.w, rd.w);
+    float4 seg = P.W.v_seg[slot];
+    int medium = __float_as_int(seg.w);
+    const bool hasval = flags & VF_HASVAL;
+    C3 value = hasval ? rgb(P.W.v_val[slot]) : cfill(0.f);
+    bool push = true;
+    {
+        float4 hv = P.W.hit[slot];
+        Hit h; h.t = hv.x; h.u = hv.y; h.v = hv.z; h.prim = __float_as_int(hv.w);
+        Frame fr = hit_frame(S, h, xyz(seg), ray.d);
+        const DevBsdf *Bp = &S.bsdfs[prim_bsdf(S, h.prim)];
+        DevBsdf Bl;
+        if (Bp->textured) {
+            Bl = *Bp;
+            tex_apply(S, Bl, hit_uv(S, h, xyz(seg), ray.d));
+            Bp = &Bl;
+        }
+        const DevBsdf &B = *Bp;
+        if (!iszero(value)) {
+            V3 to_light = xyz(P.W.v_li0[slot]);
+            float lpdf = P.W.v_li1[slot].w;
+            V3 wi = to_local(fr, to_light), wo = to_local(fr, -ray.d);
+            float ct = fabsf(wi.z);
+            float bp = P.W.v_li2[slot].w != 0.f ? 0.f : any_bsdf_pdf(B, wi, wo);
+            float w = power_heuristic(lpdf, bp);
+            L = L + (((T * value) * any_bsdf_eval(B, wi, wo)) * ct) * w;
+        }
+        BsdfRec r;
+        r.wi = to_local(fr, -ray.d); r.wo = v3(0, 0, 0);
+        r.type = BT_ALL; r.rel_eta = 1.f; r.pdf = -1.f;
+        V2 bu = next2d(rng);
+        C3 f = any_bsdf_sample(B, r, bu, rng.state);
+        if (iszero(f)) {
+            vw_done(P, slot, L);
+            push = false;
+        } else {
+            ray = make_ray(fr.p, to_world(fr, r.wo), RT_EPSILON, RT_MAX_REAL);
+            if (prim_interior(S, h.prim) != prim_exterior(S, h.prim))
+                medium = dot(fr.n, ray.d) < 0.f ? prim_interior(S, h.prim) : prim_exterior(S, h.prim);
+            P.W.bs[slot] = f4c(f, r.pdf);
+            P.W.rel_eta[slot] = r.rel_eta;
+            flags = (r.type & BT_DELTA) ? (flags | VF_DELTA) : (flags & ~VF_DELTA);
+        }
+    }
+    if (push) {
+        P.W.rng[slot] = rng;
+        P.W.rad[slot] = f4c(L, radv.w);
+        P.W.ray_o[slot] = f4(ray.o, ray.mint);
+        P.W.ray_d[slot] = f4(ray.d, ray.maxt);
+        P.W.v_seg[slot] = make_float4(seg.x, seg.y, seg.z, __int_as_float(medium));
+        P.W.flags[slot] = flags;
+    }
+    want = push ? 1u : 0u;
+    return want;
+}
 __global__ void __launch_bounds__(128, RT_VW_MINB_SAMPLE) k_vw_sample_surface(RenderParams P, int round)
 {
     round = cur_round(P, round);
@@ -674,67 +740,7 @@ __global__ void __launch_bounds__(128, RT_VW_MINB_SAMPLE) k_vw_sample_surface(Re
     VW_LOOP(C->mat[4], P.W.q_mat[4])
     {
         const int slot = VW_LIVE ? qin_[i_] : 0;
-        unsigned want = 0;
-        if (VW_LIVE) {
-        int flags = P.W.flags[slot];
-        Pcg32 rng = P.W.rng[slot];
-        float4 radv = P.W.rad[slot], tpv = P.W.tp[slot];
-        C3 L = rgb(radv), T = rgb(tpv);
-        float4 ro = P.W.ray_o[slot], rd = P.W.ray_d[slot];
-        Ray ray = make_ray(xyz(ro), xyz(rd), ro.w, rd.w);
-        float4 seg = P.W.v_seg[slot];
-        int medium = __float_as_int(seg.w);
-        const bool hasval = flags & VF_HASVAL;
-        C3 value = hasval ? rgb(P.W.v_val[slot]) : cfill(0.f);
-        bool push = true;
-        {
-            float4 hv = P.W.hit[slot];
-            Hit h; h.t = hv.x; h.u = hv.y; h.v = hv.z; h.prim = __float_as_int(hv.w);
-            Frame fr = hit_frame(S, h, xyz(seg), ray.d);
-            const DevBsdf *Bp = &S.bsdfs[prim_bsdf(S, h.prim)];
-            DevBsdf Bl;
-            if (Bp->textured) {
-                Bl = *Bp;
-                tex_apply(S, Bl, hit_uv(S, h, xyz(seg), ray.d));
-                Bp = &Bl;
-            }
-            const DevBsdf &B = *Bp;
-            if (!iszero(value)) {
-                V3 to_light = xyz(P.W.v_li0[slot]);
-                float lpdf = P.W.v_li1[slot].w;
-                V3 wi = to_local(fr, to_light), wo = to_local(fr, -ray.d);
-                float ct = fabsf(wi.z);
-                float bp = P.W.v_li2[slot].w != 0.f ? 0.f : vp_bsdf_pdf(B, wi, wo);
-                float w = power_heuristic(lpdf, bp);
-                L = L + (((T * value) * vp_bsdf_eval(B, wi, wo)) * ct) * w;
-            }
-            BsdfRec r;
-            r.wi = to_local(fr, -ray.d); r.wo = v3(0, 0, 0);
-            r.type = BT_ALL; r.rel_eta = 1.f; r.pdf = -1.f;
-            V2 bu = next2d(rng);
-            C3 f = vp_bsdf_sample(B, r, bu, rng.state);
-            if (iszero(f)) {
-                vw_done(P, slot, L);
-                push = false;
-            } else {
-                ray = make_ray(fr.p, to_world(fr, r.wo), RT_EPSILON, RT_MAX_REAL);
-                if (prim_interior(S, h.prim) != prim_exterior(S, h.prim))
-                    medium = dot(fr.n, ray.d) < 0.f ? prim_interior(S, h.prim) : prim_exterior(S, h.prim);
-                P.W.bs[slot] = f4c(f, r.pdf);
-                P.W.rel_eta[slot] = r.rel_eta;
-                flags = (r.type & BT_DELTA) ? (flags | VF_DELTA) : (flags & ~VF_DELTA);
-            }
-        }
-        if (push) {
-            P.W.rng[slot] = rng;
-            P.W.rad[slot] = f4c(L, radv.w);
-            P.W.ray_o[slot] = f4(ray.o, ray.mint);
-            P.W.ray_d[slot] = f4(ray.d, ray.maxt);
-            P.W.v_seg[slot] = make_float4(seg.x, seg.y, seg.z, __int_as_float(medium));
-            P.W.flags[slot] = flags;
-        }
-        want = push ? 1u : 0u;
-        }
+        const unsigned want = VW_LIVE ? vw_surface_path(P, S, slot) : 0u;
         q_push(out_q, out_n, slot, want);
     }
 }
@@ -820,6 +826,31 @@ __device__ __forceinline__ bool vw_finish_one(const RenderParams &P, const DevSc
 
 // k_vw_trsamp_finish: evalTransmittanceFromSampledBSDF along the ray that
 // k_vw_sample_surface sampled at a surface vertex, then vw_finish_one
+__device__ __forceinline__ unsigned vw_trsamp_path(const RenderParams &P, const DevScene &S, int slot, int &limit)
+{
+    unsigned want = 0;
+    int flags = P.W.flags[slot];
+    Pcg32 rng = P.W.rng[slot];
+    const float4 ro = P.W.ray_o[slot], rd = P.W.ray_d[slot];
+    const float4 hv = P.W.hit[slot];
+    Hit h; h.t = hv.x; h.u = hv.y; h.v = hv.z; h.prim = __float_as_int(hv.w);
+    float4 seg = P.W.v_seg[slot];
+    V3 so = xyz(seg);
+    Hit h1;
+    bool was, was1;
+    int newm = -1;
+    const C3 tr = vw_tr_sampled(S, make_ray(xyz(ro), xyz(rd), ro.w, rd.w), rng, __float_as_int(seg.w), h, so,
+                                was, h1, was1, newm, limit);
+    flags = (flags & ~VF_NEWM) | (newm >= 0 ? VF_NEWM : 0);
+    const float4 seg1 = was1 ? make_float4(ro.x, ro.y, ro.z, seg.w) : seg;
+    seg = make_float4(so.x, so.y, so.z, seg.w);
+    const float4 radv = P.W.rad[slot];
+    want = vw_finish_one<false>(P, S, slot, flags, rng, ro, rd, seg, h, was, h1, was1, seg1, tr, rgb(radv), __float_as_int(radv.w),
+                         P.W.tp[slot], P.W.bs[slot])
+               ? 1u
+               : 0u;
+    return want;
+}
 __global__ void __launch_bounds__(128, RT_VW_MINB_TRSAMP) k_vw_trsamp_finish(RenderParams P, int round)
 {
     round = cur_round(P, round);
@@ -833,29 +864,7 @@ __global__ void __launch_bounds__(128, RT_VW_MINB_TRSAMP) k_vw_trsamp_finish(Ren
     VW_LOOP(C->mat[2], P.W.q_mat[2])
     {
         const int slot = VW_LIVE ? qin_[i_] : 0;
-        unsigned want = 0;
-        if (VW_LIVE) {
-        int flags = P.W.flags[slot];
-        Pcg32 rng = P.W.rng[slot];
-        const float4 ro = P.W.ray_o[slot], rd = P.W.ray_d[slot];
-        const float4 hv = P.W.hit[slot];
-        Hit h; h.t = hv.x; h.u = hv.y; h.v = hv.z; h.prim = __float_as_int(hv.w);
-        float4 seg = P.W.v_seg[slot];
-        V3 so = xyz(seg);
-        Hit h1;
-        bool was, was1;
-        int newm = -1;
-        const C3 tr = vw_tr_sampled(S, make_ray(xyz(ro), xyz(rd), ro.w, rd.w), rng, __float_as_int(seg.w), h, so,
-                                    was, h1, was1, newm, limit);
-        flags = (flags & ~VF_NEWM) | (newm >= 0 ? VF_NEWM : 0);
-        const float4 seg1 = was1 ? make_float4(ro.x, ro.y, ro.z, seg.w) : seg;
-        seg = make_float4(so.x, so.y, so.z, seg.w);
-        const float4 radv = P.W.rad[slot];
-        want = vw_finish_one<false>(P, S, slot, flags, rng, ro, rd, seg, h, was, h1, was1, seg1, tr, rgb(radv), __float_as_int(radv.w),
-                             P.W.tp[slot], P.W.bs[slot])
-                   ? 1u
-                   : 0u;
-        }
+        const unsigned want = VW_LIVE ? vw_trsamp_path(P, S, slot, limit) : 0u;
         q_push(out_q, out_n, slot, want);
     }
     if (limit) atomicOr(P.limit_flag, RT_LIM_VOLPATH);
@@ -866,6 +875,51 @@ __global__ void __launch_bounds__(128, RT_VW_MINB_TRSAMP) k_vw_trsamp_finish(Ren
 // (the phase function's), the transmittance along it, then the light
 // sample's MIS with the phase function (no draws, so its place after the
 // transmittance leaves the path's stream as it was) and vw_finish_one
+__device__ __forceinline__ unsigned vw_scatter_path(const RenderParams &P, const DevScene &S, int slot, int &limit)
+{
+    unsigned want = 0;
+    int flags = P.W.flags[slot];
+    Pcg32 rng = P.W.rng[slot];
+    float4 seg = P.W.v_seg[slot];
+    const int medium = __float_as_int(seg.w);
+    float4 rd = P.W.ray_d[slot];
+    V3 wo;
+    float pfpdf;
+    const float pfw = phase_sample(S.media[medium], -xyz(rd), next2d(rng), wo, pfpdf);
+    const float4 ro = f4(xyz(P.W.v_p[slot]), 0.f);
+    rd = f4(wo, rd.w);
+    const float4 hv = P.W.hit[slot];
+    Hit h; h.t = hv.x; h.u = hv.y; h.v = hv.z; h.prim = __float_as_int(hv.w);
+    V3 so = xyz(seg);
+    Hit h1;
+    bool was, was1;
+    int newm = -1;
+    const C3 tr = vw_tr_sampled(S, make_ray(xyz(ro), wo, 0.f, rd.w), rng, medium, h, so, was, h1, was1, newm, limit);
+    flags = (flags & ~VF_NEWM) | (newm >= 0 ? VF_NEWM : 0);
+    const float4 seg1 = was1 ? make_float4(ro.x, ro.y, ro.z, seg.w) : seg;
+    seg = make_float4(so.x, so.y, so.z, seg.w);
+    // the light sample's MIS at the scatter point
+    const float4 radv = P.W.rad[slot], tpv = P.W.tp[slot];
+    C3 L = rgb(radv);
+    if (flags & VF_HASVAL) {
+        const C3 value = rgb(P.W.v_val[slot]);
+        if (!iszero(value)) {
+            const DevMedium &M = S.media[medium];
+            const V3 din = xyz(P.W.ray_d[slot]);
+            const V3 to_light = xyz(P.W.v_li0[slot]);
+            const float lpdf = P.W.v_li1[slot].w;
+            const float pf = P.W.v_li2[slot].w != 0.f ? 0.f : phase_eval(M, to_light, -din);
+            const float w = power_heuristic(lpdf, pf);
+            const float ev = phase_eval(M, to_light, -din);
+            L = L + ((rgb(tpv) * value) * ev) * w;
+        }
+    }
+    want = vw_finish_one<true>(P, S, slot, flags, rng, ro, rd, seg, h, was, h1, was1, seg1, tr, L,
+                         __float_as_int(radv.w), tpv, f4c(cfill(pfw), pfpdf))
+               ? 1u
+               : 0u;
+    return want;
+}
 __global__ void __launch_bounds__(128, RT_VW_MINB_TRSAMP) k_vw_scatter(RenderParams P, int round)
 {
     round = cur_round(P, round);
@@ -879,50 +933,48 @@ __global__ void __launch_bounds__(128, RT_VW_MINB_TRSAMP) k_vw_scatter(RenderPar
     VW_LOOP(C->mat[1], P.W.q_mat[1])
     {
         const int slot = VW_LIVE ? qin_[i_] : 0;
-        unsigned want = 0;
-        if (VW_LIVE) {
-        int flags = P.W.flags[slot];
-        Pcg32 rng = P.W.rng[slot];
-        float4 seg = P.W.v_seg[slot];
-        const int medium = __float_as_int(seg.w);
-        float4 rd = P.W.ray_d[slot];
-        V3 wo;
-        float pfpdf;
-        const float pfw = phase_sample(S.media[medium], -xyz(rd), next2d(rng), wo, pfpdf);
-        const float4 ro = f4(xyz(P.W.v_p[slot]), 0.f);
-        rd = f4(wo, rd.w);
-        const float4 hv = P.W.hit[slot];
-        Hit h; h.t = hv.x; h.u = hv.y; h.v = hv.z; h.prim = __float_as_int(hv.w);
-        V3 so = xyz(seg);
-        Hit h1;
-        bool was, was1;
-        int newm = -1;
-        const C3 tr = vw_tr_sampled(S, make_ray(xyz(ro), wo, 0.f, rd.w), rng, medium, h, so, was, h1, was1, newm, limit);
-        flags = (flags & ~VF_NEWM) | (newm >= 0 ? VF_NEWM : 0);
-        const float4 seg1 = was1 ? make_float4(ro.x, ro.y, ro.z, seg.w) : seg;
-        seg = make_float4(so.x, so.y, so.z, seg.w);
-        // the light sample's MIS at the scatter point
-        const float4 radv = P.W.rad[slot], tpv = P.W.tp[slot];
-        C3 L = rgb(radv);
-        if (flags & VF_HASVAL) {
-            const C3 value = rgb(P.W.v_val[slot]);
-            if (!iszero(value)) {
-                const DevMedium &M = S.media[medium];
-                const V3 din = xyz(P.W.ray_d[slot]);
-                const V3 to_light = xyz(P.W.v_li0[slot]);
-                const float lpdf = P.W.v_li1[slot].w;
-                const float pf = P.W.v_li2[slot].w != 0.f ? 0.f : phase_eval(M, to_light, -din);
-                const float w = power_heuristic(lpdf, pf);
-                const float ev = phase_eval(M, to_light, -din);
-                L = L + ((rgb(tpv) * value) * ev) * w;
-            }
-        }
-        want = vw_finish_one<true>(P, S, slot, flags, rng, ro, rd, seg, h, was, h1, was1, seg1, tr, L,
-                             __float_as_int(radv.w), tpv, f4c(cfill(pfw), pfpdf))
-                   ? 1u
-                   : 0u;
-        }
+        const unsigned want = VW_LIVE ? vw_scatter_path(P, S, slot, limit) : 0u;
         q_push(out_q, out_n, slot, want);
     }
     if (limit) atomicOr(P.limit_flag, RT_LIM_VOLPATH);
+}
+
+// Every path of the round's trace queue run to its end by one thread, the
+// wavefront's steps one after another with the path's state in memory between
+// them.  Taken for a round with at most P.tail_paths paths (tail_begin), where
+// a wavefront round is five launches that each wait for their slowest path:
+// the rounds that are left cost one launch together.  The films are the
+// wavefront's: the steps are.  Grid medium, 133x97 x 9 spp: 3.24 -> 1.78 ms.
+// (Two blocks per SM hold RT_VW_TAIL paths; 3 to 8 were 0-10 % slower.)
+#ifndef RT_VW_TAIL_MINB
+#define RT_VW_TAIL_MINB 2
+#endif
+__global__ void __launch_bounds__(128, RT_VW_TAIL_MINB) k_vw_tail(RenderParams P, int round)
+{
+    round = cur_round(P, round);
+    const DevScene &S = P.S;
+    RoundCounters *C = &P.W.cnt[round];
+    const int n = C->closest;
+    if (!tail_begin(P, C, n)) return;
+    const int *queue = vw_trace_queue(P, round);
+    int limit = 0, first, end;
+    tail_share(n, first, end);
+    for (int i = first; i < end; i += 32) {
+        const int slot = queue[i];
+        for (;;) {
+            const unsigned w = vw_step_path(P, S, slot, limit);
+            if (w == 0) break;          // the path has ended
+            if (w == 8u) continue;      // a null boundary crossed
+            bool scat = w == 2u;
+            if (w == 1u) scat = vw_shadow_path(P, S, slot, limit) == 1u;
+            if (scat) {
+                if (!vw_scatter_path(P, S, slot, limit)) break;
+            } else {
+                if (!vw_surface_path(P, S, slot)) break;
+                if (!vw_trsamp_path(P, S, slot, limit)) break;
+            }
+        }
+    }
+    if (limit) atomicOr(P.limit_flag, RT_LIM_VOLPATH);
+    tail_end(C);
 }
