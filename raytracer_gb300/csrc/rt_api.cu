@@ -1204,10 +1204,11 @@ __device__ __forceinline__ void pt_shade_path(const RenderParams &P, const DevSc
     V3 o = xyz(ro), d = xyz(rd);
     float4 hv = P.W.hit[slot];
     Hit h; h.t = hv.x; h.u = hv.y; h.v = hv.z; h.prim = __float_as_int(hv.w);
-    Frame fr = hit_frame(S, h, o, d);
+    int hit_bsdf, hit_light;
+    Frame fr = hit_frame(S, h, o, d, hit_bsdf, hit_light);
     // a textured BSDF (mixed queue only) is a copy with its textures applied
     // at the hit
-    const DevBsdf *Bp = &S.bsdfs[prim_bsdf(S, h.prim)];
+    const DevBsdf *Bp = &S.bsdfs[hit_bsdf];
     DevBsdf Bl;
     if (BT == RT_QUEUE_MIXED && Bp->textured) {
         Bl = *Bp;
@@ -1226,7 +1227,7 @@ __device__ __forceinline__ void pt_shade_path(const RenderParams &P, const DevSc
         flags &= ~F_NEE;
         float4 bsv = P.W.bs[slot];
         C3 f = rgb(bsv);
-        int nl = prim_light(S, h.prim);
+        const int nl = hit_light;
         if (nl >= 0) {
             C3 Le = area_le(S, nl, -d, fr.n);
             float pl = (flags & F_DELTA) ? 0.f : light_pdf(S, nl, o, fr.p, fr.n, d);
@@ -1252,8 +1253,7 @@ __device__ __forceinline__ void pt_shade_path(const RenderParams &P, const DevSc
     } else {
     // emission of a light hit by the camera ray (PathTracingMIS.cpp:73-74)
     if (depth == 0) {
-        int hl = prim_light(S, h.prim);
-        if (hl >= 0) L = L + T * area_le(S, hl, -d, fr.n);
+        if (hit_light >= 0) L = L + T * area_le(S, hit_light, -d, fr.n);
     }
     // light sampling (Integrator::sampleLightDirect, Integrator.cpp:176-218)
     if (ALL) {
@@ -1659,23 +1659,23 @@ __global__ void k_film_wide(RenderParams P, float4 *film, int t0, int t1, int ti
 // rt_scene_refit: new vertex positions into the triangle arrays, then the
 // binary tree's boxes bottom-up over its unchanged topology, widened as the
 // host build widens them, then the 4-wide tree's copies of them.
-__global__ void k_refit_tris(const float *vtx, const float *nrm, const int32_t *idx, int nt, float *tri_v, float *tri_n)
+__global__ void k_refit_tris(const float *vtx, const float *nrm, const int32_t *idx, int nt, float4 *tri_rec, float *tri_n)
 {
     for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < nt; t += gridDim.x * blockDim.x)
         for (int k = 0; k < 3; k++) {
             const size_t v = (size_t)idx[3 * (size_t)t + k];
-            for (int a = 0; a < 3; a++) {
-                tri_v[9 * (size_t)t + 3 * k + a] = vtx[3 * v + a];
-                if (tri_n) tri_n[9 * (size_t)t + 3 * k + a] = nrm[3 * v + a];
-            }
+            float4 &R = tri_rec[3 * (size_t)t + k];
+            R = make_float4(vtx[3 * v], vtx[3 * v + 1], vtx[3 * v + 2], R.w);
+            for (int a = 0; a < 3 && tri_n; a++) tri_n[9 * (size_t)t + 3 * k + a] = nrm[3 * v + a];
         }
 }
 // triangle slots (p0 and id, e1 = p1 - p0, e2 = p2 - p0) from the new vertices
-__global__ void k_refit_slots(float4 *slots, int n_slots, const float *tri_v)
+__global__ void k_refit_slots(float4 *slots, int n_slots, const float4 *tri_rec)
 {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n_slots; i += gridDim.x * blockDim.x) {
         const float4 a = slots[3 * (size_t)i];
-        const float *P = tri_v + 9 * (size_t)__float_as_int(a.w);
+        float P[9];
+        tri_load(tri_rec, __float_as_int(a.w), P);
         slots[3 * (size_t)i] = make_float4(P[0], P[1], P[2], a.w);
         slots[3 * (size_t)i + 1] = make_float4(P[3] - P[0], P[4] - P[1], P[5] - P[2], 0.f);
         slots[3 * (size_t)i + 2] = make_float4(P[6] - P[0], P[7] - P[1], P[8] - P[2], 0.f);
@@ -1684,7 +1684,7 @@ __global__ void k_refit_slots(float4 *slots, int n_slots, const float *tri_v)
 // one level of internal nodes: the exact boxes of both children (a leaf's
 // triangles, or an internal child's two boxes from the deeper level) into
 // boxes[12 * node]: child 0 then child 1, each (min xyz, max xyz)
-__global__ void k_refit_level(const float4 *nodes, const float4 *slots, const float *tri_v, const int32_t *order,
+__global__ void k_refit_level(const float4 *nodes, const float4 *slots, const float4 *tri_rec, const int32_t *order,
                               int begin, int end, float *boxes)
 {
     for (int i = begin + blockIdx.x * blockDim.x + threadIdx.x; i < end; i += gridDim.x * blockDim.x) {
@@ -1702,7 +1702,8 @@ __global__ void k_refit_level(const float4 *nodes, const float4 *slots, const fl
             } else if (link < 0) {
                 const int v = ~link, first = v >> 3, cnt = (v & 7) + 1;
                 for (int j = 0; j < cnt; j++) {
-                    const float *P = tri_v + 9 * (size_t)__float_as_int(slots[3 * (size_t)(first + j)].w);
+                    float P[9];
+                    tri_load(tri_rec, __float_as_int(slots[3 * (size_t)(first + j)].w), P);
                     for (int c = 0; c < 3; c++)
                         for (int a = 0; a < 3; a++) {
                             b[a] = fminf(b[a], P[3 * c + a]);
@@ -2450,7 +2451,7 @@ static rt_status validate(const rt_scene_desc *d)
 static rt_status launch_check(const char *what);
 
 // The binary tree built on the device (rt_lbvh.cuh) over the scene's
-// triangles, already on the device in S.tri_v: the node image and the
+// triangles, already on the device in S.tri_rec: the node image and the
 // triangle slots, in memory the scene owns.  RT_ERR_LIMIT when the tree is
 // deeper than the traversal stacks (the caller then builds on the host).
 static rt_status device_tree(rt_ctx *ctx, rt_scene *sc, int nt)
@@ -2489,7 +2490,7 @@ static rt_status device_tree(rt_ctx *ctx, rt_scene *sc, int nt)
         const float ext = sc->bounds[3 + a] - sc->bounds[a];
         scale[a] = ext > 0.f ? 1024.f / ext : 0.f;
     }
-    k_lbvh_codes<<<grid(nt), 256, 0, st>>>(S.tri_v, nt, sc->bounds[0], sc->bounds[1], sc->bounds[2], scale[0], scale[1],
+    k_lbvh_codes<<<grid(nt), 256, 0, st>>>(S.tri_rec, nt, sc->bounds[0], sc->bounds[1], sc->bounds[2], scale[0], scale[1],
                                           scale[2], code[0], id[0]);
     int cur = 0;
     for (int shift = 0; shift < 30; shift += 8) {
@@ -2502,9 +2503,9 @@ static rt_status device_tree(rt_ctx *ctx, rt_scene *sc, int nt)
     k_lbvh_nodes<<<grid(nt - 1), 256, 0, st>>>(code[cur], nt, nodes, ipar, lpar);
     if (cudaMemsetAsync(arr, 0, 4 * n, st) != cudaSuccess || cudaMemsetAsync(depth, 0, 4, st) != cudaSuccess)
         return done(fail(RT_ERR_CUDA, "device tree: memset failed"));
-    k_lbvh_boxes<<<grid(nt), 256, 0, st>>>(S.tri_v, id[cur], nt, ipar, lpar, arr, boxes, depth);
+    k_lbvh_boxes<<<grid(nt), 256, 0, st>>>(S.tri_rec, id[cur], nt, ipar, lpar, arr, boxes, depth);
     k_refit_widen<<<grid(nt - 1), 256, 0, st>>>(nodes, nt - 1, boxes);
-    k_lbvh_slots<<<grid(nt), 256, 0, st>>>(S.tri_v, id[cur], nt, slots);
+    k_lbvh_slots<<<grid(nt), 256, 0, st>>>(S.tri_rec, id[cur], nt, slots);
     if ((s = launch_check("device tree kernels")) != RT_OK) return done(s);
     int maxd = 0;
     if (cudaMemcpyAsync(&maxd, depth, 4, cudaMemcpyDeviceToHost, st) != cudaSuccess || cudaStreamSynchronize(st) != cudaSuccess)
@@ -2723,8 +2724,12 @@ static rt_status scene_create(rt_ctx *ctx, const rt_scene_desc *d, const ExtTree
             V3 c = 0.5f * (bmx + bmn);
             D.env_radius = 2 * h_smax(norm(bmn - c), norm(bmx - c));
             const float *dp;
-            if ((st = upload(sc, L.env_rgb, 3 * (size_t)Wd * H, &dp)) != RT_OK) { rt_scene_destroy(sc); return st; }
-            D.env_rgb = dp;
+            std::vector<float4> texels((size_t)Wd * H);
+            for (size_t i = 0; i < texels.size(); i++)
+                texels[i] = make_float4(L.env_rgb[3 * i], L.env_rgb[3 * i + 1], L.env_rgb[3 * i + 2], 0.f);
+            const float4 *tp4;
+            if ((st = upload(sc, texels.data(), texels.size(), &tp4)) != RT_OK) { rt_scene_destroy(sc); return st; }
+            D.env_rgb = tp4;
             if ((st = upload(sc, rows.data(), rows.size(), &dp)) != RT_OK) { rt_scene_destroy(sc); return st; }
             D.env_row_cdf = dp;
             if ((st = upload(sc, marg.c.data(), marg.c.size(), &dp)) != RT_OK) { rt_scene_destroy(sc); return st; }
@@ -2764,9 +2769,22 @@ static rt_status scene_create(rt_ctx *ctx, const rt_scene_desc *d, const ExtTree
         media[m].density = dp;
     }
     const float *fp;
-    const int *ip;
-    if ((st = upload(sc, tri_v.data(), tri_v.size(), &fp)) != RT_OK) { rt_scene_destroy(sc); return st; }
-    S.tri_v = fp;
+    {
+        std::vector<float4> rec(3 * (size_t)nt);
+        for (int t = 0; t < nt; t++) {
+            const int m = tri_mesh[t];
+            const int ids[3] = {m < d->n_meshes ? d->meshes[m].bsdf : -1, m < d->n_meshes ? d->meshes[m].light : -1, m};
+            for (int k = 0; k < 3; k++) {
+                const float *p = &tri_v[9 * (size_t)t + 3 * k];
+                float w;
+                std::memcpy(&w, &ids[k], 4);
+                rec[3 * (size_t)t + k] = make_float4(p[0], p[1], p[2], w);
+            }
+        }
+        const float4 *rp;
+        if ((st = upload(sc, rec.data(), rec.size(), &rp)) != RT_OK) { rt_scene_destroy(sc); return st; }
+        S.tri_rec = rp;
+    }
     // BVH: built on the device when the context asks for it (a tree too deep
     // for the stacks falls back to the host build), else on the host
     bool dev_tree = false;
@@ -2898,8 +2916,6 @@ static rt_status scene_create(rt_ctx *ctx, const rt_scene_desc *d, const ExtTree
         S.has_textured |= b.textured;
         S.has_mixed |= bsdf_queue_of(b) == RT_QUEUE_MIXED;
     }
-    if ((st = upload(sc, tri_mesh.data(), tri_mesh.size(), &ip)) != RT_OK) { rt_scene_destroy(sc); return st; }
-    S.tri_mesh = ip;
     {
         // BSDF type per triangle: the closest-hit trace sorts hits by it
         std::vector<uint8_t> tri_type(nt, 255);
@@ -3058,12 +3074,12 @@ rt_status rt_scene_refit(rt_ctx *ctx, rt_scene *sc, const float *vertices, const
     }
     const int sm = ctx->sm_count > 0 ? ctx->sm_count : 1;
     auto grid = [&](int64_t n) { return (int)std::max<int64_t>(1, std::min<int64_t>((n + 255) / 256, (int64_t)sm * 16)); };
-    k_refit_tris<<<grid(n_tris), 256, 0, st>>>(vd, nd_, sc->indices_dev, n_tris, const_cast<float *>(sc->S.tri_v),
+    k_refit_tris<<<grid(n_tris), 256, 0, st>>>(vd, nd_, sc->indices_dev, n_tris, const_cast<float4 *>(sc->S.tri_rec),
                                                const_cast<float *>(sc->S.tri_n));
-    k_refit_slots<<<grid(n_tris), 256, 0, st>>>(const_cast<float4 *>(sc->S.tri_slots), n_tris, sc->S.tri_v);
+    k_refit_slots<<<grid(n_tris), 256, 0, st>>>(const_cast<float4 *>(sc->S.tri_slots), n_tris, sc->S.tri_rec);
     for (size_t l = 0; l + 1 < sc->level_off.size(); l++) {
         const int b = sc->level_off[l], e = sc->level_off[l + 1];
-        k_refit_level<<<grid(e - b), 256, 0, st>>>(sc->S.nodes, sc->S.tri_slots, sc->S.tri_v, sc->refit_order, b, e,
+        k_refit_level<<<grid(e - b), 256, 0, st>>>(sc->S.nodes, sc->S.tri_slots, sc->S.tri_rec, sc->refit_order, b, e,
                                                     sc->refit_boxes);
     }
     k_refit_widen<<<grid(sc->S.n_nodes), 256, 0, st>>>(const_cast<float4 *>(sc->S.nodes), sc->S.n_nodes, sc->refit_boxes);

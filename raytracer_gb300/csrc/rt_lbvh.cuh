@@ -40,11 +40,12 @@ __device__ __forceinline__ unsigned lbvh_expand10(unsigned v)
     return v;
 }
 
-__global__ void k_lbvh_codes(const float *tri_v, int n, float bx0, float by0, float bz0, float sx, float sy, float sz,
+__global__ void k_lbvh_codes(const float4 *tri_rec, int n, float bx0, float by0, float bz0, float sx, float sy, float sz,
                              unsigned *codes, int *ids)
 {
     for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
-        const float *P = tri_v + 9 * (size_t)t;
+        float P[9];
+        tri_load(tri_rec, t, P);
         const float c[3] = {(P[0] + P[3] + P[6]) * (1.f / 3.f), (P[1] + P[4] + P[7]) * (1.f / 3.f),
                             (P[2] + P[5] + P[8]) * (1.f / 3.f)};
         const float o[3] = {bx0, by0, bz0}, sc[3] = {sx, sy, sz};
@@ -190,11 +191,12 @@ __global__ void k_lbvh_nodes(const unsigned *codes, int n, float4 *nodes, int *i
 
 // boxes from the leaves up: every leaf writes its triangle's box into its
 // parent's child slot; the second arrival at a node unites the two and goes on
-__global__ void k_lbvh_boxes(const float *tri_v, const int *ids, int n, const int *iparent, const int *lparent,
+__global__ void k_lbvh_boxes(const float4 *tri_rec, const int *ids, int n, const int *iparent, const int *lparent,
                              int *arrivals, float *boxes, int *max_depth)
 {
     for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < n; s += gridDim.x * blockDim.x) {
-        const float *P = tri_v + 9 * (size_t)ids[s];
+        float P[9];
+        tri_load(tri_rec, ids[s], P);
         float b[6];
         for (int a = 0; a < 3; a++) {
             b[a] = fminf(fminf(P[a], P[3 + a]), P[6 + a]);
@@ -230,11 +232,12 @@ __global__ void k_lbvh_boxes(const float *tri_v, const int *ids, int n, const in
 }
 
 // triangle slots in sorted order: (p0, id), (p1 - p0), (p2 - p0)
-__global__ void k_lbvh_slots(const float *tri_v, const int *ids, int n, float4 *slots)
+__global__ void k_lbvh_slots(const float4 *tri_rec, const int *ids, int n, float4 *slots)
 {
     for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < n; s += gridDim.x * blockDim.x) {
         const int id = ids[s];
-        const float *P = tri_v + 9 * (size_t)id;
+        float P[9];
+        tri_load(tri_rec, id, P);
         slots[3 * (size_t)s] = make_float4(P[0], P[1], P[2], __int_as_float(id));
         slots[3 * (size_t)s + 1] = make_float4(P[3] - P[0], P[4] - P[1], P[5] - P[2], 0.f);
         slots[3 * (size_t)s + 2] = make_float4(P[6] - P[0], P[7] - P[1], P[8] - P[2], 0.f);
