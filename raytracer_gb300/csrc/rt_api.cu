@@ -205,12 +205,10 @@ __global__ void k_camera(RenderParams P)
             P.W.splat[slot] = code;
             if (code != 0x55) P.W.pix_irregular[q] = 1;
         }
-        P.W.rng[slot] = rng;
-        P.W.ray_o[slot] = f4(r.o, r.mint);
-        P.W.ray_d[slot] = f4(r.d, r.maxt);
-        P.W.tp[slot] = make_float4(1.f, 1.f, 1.f, 1.f);
-        P.W.rad[slot] = make_float4(0.f, 0.f, 0.f, __int_as_float(0));
-        P.W.flags[slot] = F_FIRST;
+        const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+        w_store2(P.W.ray, slot, f4(r.o, r.mint), f4(r.d, r.maxt));
+        w_store2(P.W.acc, slot, make_float4(1.f, 1.f, 1.f, 1.f), zero);
+        w_store2(P.W.smp, slot, zero, path_rng_pack(rng, F_FIRST));
         P.W.q_closest[slot] = slot;
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -254,12 +252,10 @@ __global__ void k_camera_multi(RenderParams P)
         P.W.splat[slot] = code;
         if (code != 0x55) P.W.pix_irregular[it.pix0 + q] = 1;
         P.W.sid[slot] = it.job;
-        P.W.rng[slot] = rng;
-        P.W.ray_o[slot] = f4(r.o, r.mint);
-        P.W.ray_d[slot] = f4(r.d, r.maxt);
-        P.W.tp[slot] = make_float4(1.f, 1.f, 1.f, 1.f);
-        P.W.rad[slot] = make_float4(0.f, 0.f, 0.f, __int_as_float(0));
-        P.W.flags[slot] = F_FIRST;
+        const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+        w_store2(P.W.ray, slot, f4(r.o, r.mint), f4(r.d, r.maxt));
+        w_store2(P.W.acc, slot, make_float4(1.f, 1.f, 1.f, 1.f), zero);
+        w_store2(P.W.smp, slot, zero, path_rng_pack(rng, F_FIRST));
         P.W.q_closest[slot] = slot;
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -298,8 +294,12 @@ __device__ __forceinline__ int trace_fetch(const Wave &W, const int *queue, int 
     const int q = base + __popc(m & ((1u << lane) - 1));
     if (!want || q >= n) return -1;
     const int slot = queue[q];
-    o = ANY ? W.sh_o[slot] : W.ray_o[slot];
-    d = ANY ? W.sh_d[slot] : W.ray_d[slot];
+    if (ANY) {
+        o = w_ray_o(W, slot);
+        d = w_sh_d(W, slot);
+    } else {
+        w_load2(W.ray, slot, o, d);
+    }
     return slot;
 }
 
@@ -344,8 +344,8 @@ __global__ void k_sort_count(RenderParams P, int round, int shadow)
     const int *queue = shadow ? P.W.q_shadow : P.W.q_closest;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         int slot = queue[i];
-        float4 o = shadow ? P.W.sh_o[slot] : P.W.ray_o[slot];
-        float4 d = shadow ? P.W.sh_d[slot] : P.W.ray_d[slot];
+        float4 o = w_ray_o(P.W, slot);
+        float4 d = shadow ? w_sh_d(P.W, slot) : w_ray_d(P.W, slot);
         unsigned k = ray_sort_key(P.S, o, d);
         P.W.sort_keys[i] = k;
         atomicAdd(&P.W.sort_hist[k], 1u);
@@ -569,7 +569,7 @@ __global__ void __launch_bounds__(128, RT_TRACE_MINB) k_trace(RenderParams P, in
                     }
                 }
             }
-            if (ANY) P.W.occl[slot] = hprim != -1 ? 1 : 0;
+            if (ANY) w_set_occluded(P.W, slot, hprim != -1);
             else {
                 P.W.hit[slot] = make_float4(hit_t, hu, hv, __int_as_float(hprim));
                 to_queue = MULTI ? hit_queue(P, *ms, hprim, n) : hit_queue(P, S, hprim, n);
@@ -751,7 +751,7 @@ __global__ void __launch_bounds__(128, RT_TRACE4_MINB) k_trace4(RenderParams P, 
                     }
                 }
             }
-            if (ANY) P.W.occl[slot] = hprim != -1 ? 1 : 0;
+            if (ANY) w_set_occluded(P.W, slot, hprim != -1);
             else {
                 P.W.hit[slot] = make_float4(hit_t, hu, hv, __int_as_float(hprim));
                 to_queue = hit_queue(P, S, hprim, n);
@@ -954,7 +954,7 @@ __global__ void __launch_bounds__(128, 8) k_trace8(RenderParams P, int round)
                     }
                 }
             }
-            if (ANY) P.W.occl[slot] = hprim != -1 ? 1 : 0;
+            if (ANY) w_set_occluded(P.W, slot, hprim != -1);
             else {
                 P.W.hit[slot] = make_float4(hit_t, hu, hv, __int_as_float(hprim));
                 to_queue = hit_queue(P, S, hprim, n);
@@ -984,8 +984,9 @@ __global__ void k_rays_in(const rt_ray *rays, int n, RenderParams P, int anyhit)
     if (i >= n) return;
     rt_ray r = rays[i];
     float4 o = make_float4(r.o[0], r.o[1], r.o[2], r.mint), d = make_float4(r.d[0], r.d[1], r.d[2], r.maxt);
-    if (anyhit) { P.W.sh_o[i] = o; P.W.sh_d[i] = d; P.W.q_shadow[i] = i; }
-    else { P.W.ray_o[i] = o; P.W.ray_d[i] = d; P.W.q_closest[i] = i; }
+    w_ray_o(P.W, i) = o;
+    if (anyhit) { w_sh_d(P.W, i) = d; P.W.q_shadow[i] = i; }
+    else { w_ray_d(P.W, i) = d; P.W.q_closest[i] = i; }
     if (i == 0) {
         RoundCounters c;
         memset(&c, 0, sizeof(c));
@@ -1000,7 +1001,7 @@ __global__ void k_hits_out(RenderParams P, int n, int anyhit, rt_hit *hits)
     if (i >= n) return;
     rt_hit h;
     if (anyhit) {
-        h.t = 0.f; h.u = 0.f; h.v = 0.f; h.prim = P.W.occl[i] ? 0 : -1;
+        h.t = 0.f; h.u = 0.f; h.v = 0.f; h.prim = __float_as_int(w_nee(P.W, i).w) ? 0 : -1;
     } else {
         float4 v = P.W.hit[i];
         int prim = __float_as_int(v.w);
@@ -1030,19 +1031,22 @@ __global__ void k_hits_out(RenderParams P, int n, int anyhit, rt_hit *hits)
 __device__ __forceinline__ void pt_finish_path(const RenderParams &P, const DevScene &S, int slot)
 {
     const int env = S.env_light;
-    int flags = P.W.flags[slot];
-    C3 L = rgb(P.W.rad[slot]);
+    const int flags = (int)(__float_as_uint(w_rng(P.W, slot).w) & 0x7fffffffu);
+    C3 L = rgb(w_rad(P.W, slot));
     if (flags & F_FIRST) {
         // camera ray: the environment if it missed; a surface without a
         // BSDF ends the path (PathTracingMIS.cpp:60-70)
         float4 hv = P.W.hit[slot];
-        if (__float_as_int(hv.w) == -1 && env >= 0) L = L + env_le(S.lights[env], xyz(P.W.ray_d[slot]));
+        if (__float_as_int(hv.w) == -1 && env >= 0) L = L + env_le(S.lights[env], xyz(w_ray_d(P.W, slot)));
     } else {
-        if ((flags & F_NEE) && !P.W.occl[slot]) L = L + rgb(P.W.nee[slot]);
+        if (flags & F_NEE) {
+            const float4 nee = w_nee(P.W, slot);
+            if (!__float_as_int(nee.w)) L = L + rgb(nee);
+        }
         if (!(flags & F_END)) {
             float4 hv = P.W.hit[slot];
             Hit h; h.t = hv.x; h.u = hv.y; h.v = hv.z; h.prim = __float_as_int(hv.w);
-            float4 ro = P.W.ray_o[slot], rd = P.W.ray_d[slot];
+            float4 ro = w_ray_o(P.W, slot), rd = w_ray_d(P.W, slot);
             V3 o = xyz(ro), d = xyz(rd);
             int caught = -1;
             C3 Le = cfill(0.f);
@@ -1060,16 +1064,15 @@ __device__ __forceinline__ void pt_finish_path(const RenderParams &P, const DevS
                 Le = env_le(S.lights[env], d);
             }
             if (caught >= 0) {
-                C3 T = rgb(P.W.tp[slot]);
-                float4 bsv = P.W.bs[slot];
+                C3 T = rgb(w_tp(P.W, slot));
+                float4 bsv = w_bs(P.W, slot);
                 float pl = (flags & F_DELTA) ? 0.f : light_pdf(S, caught, o, pt, nn, d);
                 float w = power_heuristic(bsv.w, pl);
                 L = L + ((T * Le) * rgb(bsv)) * w;
             }
         }
     }
-    P.W.out[slot] = f4c(L, 0.f);
-    P.W.flags[slot] = (flags & ~(F_FIRST | F_NEE)) | F_DONE;
+    w_done(P.W, slot, L);
 }
 // MULTI: a multi-scene batch, each path read against its own scene
 template <bool MULTI = false>
@@ -1192,17 +1195,18 @@ template <int BT, bool ALL = false>
 __device__ __forceinline__ void pt_shade_path(const RenderParams &P, const DevScene &S, int slot, bool &push_end,
                                               bool &push_closest, bool &push_shadow)
 {
-    Pcg32 rng = P.W.rng[slot];
-    float4 tpv = P.W.tp[slot];
+    const float4 hv = P.W.hit[slot];
+    float4 ro, rd, bsv, rv, tpv, radv;
+    w_load2(P.W.ray, slot, ro, rd);
+    w_load2(P.W.smp, slot, bsv, rv);
+    w_load2(P.W.acc, slot, tpv, radv);
+    int flags;
+    Pcg32 rng = path_rng(rv, flags);
     C3 T = rgb(tpv);
     float eta = tpv.w;
-    float4 radv = P.W.rad[slot];
     C3 L = rgb(radv);
     int depth = __float_as_int(radv.w);
-    int flags = P.W.flags[slot];
-    float4 ro = P.W.ray_o[slot], rd = P.W.ray_d[slot];
     V3 o = xyz(ro), d = xyz(rd);
-    float4 hv = P.W.hit[slot];
     Hit h; h.t = hv.x; h.u = hv.y; h.v = hv.z; h.prim = __float_as_int(hv.w);
     int hit_bsdf, hit_light;
     Frame fr = hit_frame(S, h, o, d, hit_bsdf, hit_light);
@@ -1223,9 +1227,11 @@ __device__ __forceinline__ void pt_shade_path(const RenderParams &P, const DevSc
         flags &= ~F_FIRST;
         if (depth >= P.max_depth) done = true;
     } else {
-        if ((flags & F_NEE) && !P.W.occl[slot]) L = L + rgb(P.W.nee[slot]);
+        if (flags & F_NEE) {
+            const float4 nee = w_nee(P.W, slot);
+            if (!__float_as_int(nee.w)) L = L + rgb(nee);
+        }
         flags &= ~F_NEE;
-        float4 bsv = P.W.bs[slot];
         C3 f = rgb(bsv);
         const int nl = hit_light;
         if (nl >= 0) {
@@ -1235,7 +1241,6 @@ __device__ __forceinline__ void pt_shade_path(const RenderParams &P, const DevSc
             L = L + ((T * Le) * f) * w;
         }
         T = T * f;
-        eta *= P.W.rel_eta[slot];
         if (depth >= P.min_depth) {
             float stop = smin(0.95f, lum(T) * eta * eta);
             if (next1d(rng) < stop) T = T / stop;
@@ -1247,9 +1252,7 @@ __device__ __forceinline__ void pt_shade_path(const RenderParams &P, const DevSc
         }
     }
     if (done) {
-        P.W.out[slot] = f4c(L, 0.f);
-        P.W.flags[slot] = flags | F_DONE;
-        P.W.rng[slot] = rng;
+        w_done(P.W, slot, L);
     } else {
     // emission of a light hit by the camera ray (PathTracingMIS.cpp:73-74)
     if (depth == 0) {
@@ -1281,9 +1284,7 @@ __device__ __forceinline__ void pt_shade_path(const RenderParams &P, const DevSc
                 // exactly zero (e.g. a light direction below an opaque
                 // surface) its outcome cannot change L and it is not traced.
                 if (contrib.r != 0.f || contrib.g != 0.f || contrib.b != 0.f) {
-                    P.W.nee[slot] = f4c(contrib, 0.f);
-                    P.W.sh_o[slot] = f4(fr.p, RT_EPSILON);
-                    P.W.sh_d[slot] = f4(li.to_light, li.distance - RT_EPSILON);
+                    w_store2(P.W.sh, slot, f4(li.to_light, li.distance - RT_EPSILON), f4c(contrib, 0.f));
                     flags |= F_NEE;
                     push_shadow = true;
                 }
@@ -1297,26 +1298,26 @@ __device__ __forceinline__ void pt_shade_path(const RenderParams &P, const DevSc
     r.type = BT_ALL; r.rel_eta = 1.f; r.pdf = -1.f;
     V2 u = next2d(rng);
     C3 f = bsdf_sample_t<BT>(B, r, u, rng.state);
-    if (iszero(f)) {
-        if (flags & F_NEE) {
-            flags |= F_END;   // the light sample still needs its shadow ray
-            push_end = true;
-        } else {
-            flags |= F_DONE;
-            P.W.out[slot] = f4c(L, 0.f);
-        }
+    const bool ends = iszero(f);
+    if (ends && !(flags & F_NEE)) {
+        w_done(P.W, slot, L);
+        return;
+    }
+    // the next ray, and the origin of the light sample's shadow ray
+    float4 next_d = rd, next_bs = bsv;
+    if (ends) {
+        flags |= F_END;   // the light sample still needs its shadow ray
+        push_end = true;
     } else {
-        P.W.ray_o[slot] = f4(fr.p, RT_EPSILON);
-        P.W.ray_d[slot] = f4(to_world(fr, r.wo), RT_MAX_REAL);
-        P.W.bs[slot] = f4c(f, r.pdf);
-        P.W.rel_eta[slot] = r.rel_eta;
+        next_d = f4(to_world(fr, r.wo), RT_MAX_REAL);
+        next_bs = f4c(f, r.pdf);
+        eta *= r.rel_eta;   // as the next vertex reads it
         if (r.type & BT_DELTA) flags |= F_DELTA; else flags &= ~F_DELTA;
         push_closest = true;
     }
-    P.W.rad[slot] = f4c(L, __int_as_float(depth));
-    P.W.tp[slot] = f4c(T, eta);
-    P.W.rng[slot] = rng;
-    P.W.flags[slot] = flags;
+    w_store2(P.W.ray, slot, f4(fr.p, RT_EPSILON), next_d);
+    w_store2(P.W.smp, slot, next_bs, path_rng_pack(rng, flags));
+    w_store2(P.W.acc, slot, f4c(T, eta), f4c(L, __int_as_float(depth)));
     }
 }
 // MULTI: a multi-scene batch, each path shaded against its own scene.
@@ -1413,16 +1414,16 @@ __global__ void __launch_bounds__(128, RT_PT_TAIL_MINB) k_pt_tail(RenderParams P
         const int slot = i < nc ? P.W.q_closest[i] : P.W.q_end[i - nc];
         const DevScene &S = MULTI ? P.scenes[P.W.sid[slot]] : P.S;
         for (;;) {
-            const int flags = P.W.flags[slot];
+            const int flags = (int)(__float_as_uint(w_rng(P.W, slot).w) & 0x7fffffffu);
             Hit h;
             if (flags & F_NEE) {
-                const float4 o = P.W.sh_o[slot], d = P.W.sh_d[slot];
-                P.W.occl[slot] = trace_ray<true>(S, xyz(o), xyz(d), o.w, d.w, h) ? 1 : 0;
+                const float4 o = w_ray_o(P.W, slot), d = w_sh_d(P.W, slot);
+                w_set_occluded(P.W, slot, trace_ray<true>(S, xyz(o), xyz(d), o.w, d.w, h));
                 n_shadow++;
             }
             bool finish = (flags & F_END) != 0;
             if (!finish) {
-                const float4 o = P.W.ray_o[slot], d = P.W.ray_d[slot];
+                const float4 o = w_ray_o(P.W, slot), d = w_ray_d(P.W, slot);
                 h.t = d.w; h.u = h.v = 0.f;
                 trace_ray<false>(S, xyz(o), xyz(d), o.w, d.w, h);
                 P.W.hit[slot] = make_float4(h.t, h.u, h.v, __int_as_float(h.prim));
@@ -1525,17 +1526,17 @@ __device__ __forceinline__ FilmSum film_gather(const RenderParams &P, const uint
             if (!self && !irr) continue;
             const int slot = path0 + qs * spp;
             if (!irr) {
-                const float4 *L = P.W.out + slot;
+                const float4 *L = P.W.acc + 2 * (size_t)slot + 1;
                 int s = 0;
-                for (; s + 4 <= spp; s += 4) {   // a thread's sectors whole: two samples each
-                    const float4 a = __ldcs(L + s), b = __ldcs(L + s + 1), c = __ldcs(L + s + 2), d = __ldcs(L + s + 3);
+                for (; s + 4 <= spp; s += 4, L += 8) {
+                    const float4 a = __ldcs(L), b = __ldcs(L + 2), c = __ldcs(L + 4), d = __ldcs(L + 6);
                     film_add(f, a, true); film_add(f, b, true); film_add(f, c, true); film_add(f, d, true);
                 }
-                for (; s < spp; s++) film_add(f, __ldcs(L + s), true);
+                for (; s < spp; s++, L += 2) film_add(f, __ldcs(L), true);
                 continue;
             }
             for (int s = 0; s < spp; s++)
-                if (splat_covers(P.W.splat[slot + s], -dx, -dy)) film_add(f, P.W.out[slot + s], self);
+                if (splat_covers(P.W.splat[slot + s], -dx, -dy)) film_add(f, w_rad(P.W, slot + s), self);
         }
     }
     return f;
@@ -1632,7 +1633,7 @@ __global__ void k_film_wide(RenderParams P, float4 *film, int t0, int t1, int ti
                 for (int qx = qx0; qx <= qx1; qx++) {
                     const int q = tile_first - P.g0 + (qy - oy) * tw + (qx - ox);
                     for (int sm = 0; sm < P.spp; sm++) {
-                        float4 L = P.W.out[(size_t)q * P.spp + sm];
+                        float4 L = w_rad(P.W, q * P.spp + sm);
                         if (isnan(L.x) || isnan(L.y) || isnan(L.z)) continue;
                         Pcg32 rng;
                         path_stream_seed(rng, P.seed, (uint32_t)(qy * W + qx), (uint32_t)(P.sample_begin + sm));
@@ -3125,10 +3126,10 @@ static rt_status ensure_vw(rt_ctx *c, int capacity)
     if (c->W.vw_capacity >= capacity) return RT_OK;
     Wave &W = c->W;
     const size_t P = (size_t)capacity;
-    float4 **arr[6] = {&W.v_seg, &W.v_p, &W.v_li0, &W.v_li1, &W.v_li2, &W.v_val};
+    float4 **arr[3] = {&W.v_light, &W.v_point, &W.v_val};
     for (float4 **a : arr) {
         void *p = nullptr;
-        if (cudaMalloc(&p, P * sizeof(float4)) != cudaSuccess) {
+        if (cudaMalloc(&p, 2 * P * sizeof(float4)) != cudaSuccess) {
             cudaGetLastError();
             return fail(RT_ERR_NOMEM, "VolPath wavefront buffer allocation failed");
         }
@@ -3139,18 +3140,22 @@ static rt_status ensure_vw(rt_ctx *c, int capacity)
     return RT_OK;
 }
 
-// the per-slot allocations of ensure_wave and (VolPathTracing) ensure_vw
+// What a server budgets per slot: the fields of the path state, each counted
+// by itself.  The arrays of ensure_wave and (VolPathTracing) ensure_vw take 28
+// bytes less (the shadow ray's origin, the eta of the pending sample and half
+// of the stream's increment are not stored); the figure stays, so that what a
+// budget admits does.
 extern "C" int64_t rt_path_state_bytes(int32_t integrator)
 {
     if (integrator != RT_INTEGRATOR_PATH_MIS && integrator != RT_INTEGRATOR_VOLPATH) return 0;
     const bool volpath = integrator == RT_INTEGRATOR_VOLPATH;
     const int64_t wave = sizeof(Pcg32) +
-                         10 * sizeof(float4) +                 // tp rad ray_o ray_d hit bs nee sh_o sh_d out
-                         3 * sizeof(int) +                     // rel_eta flags occl
+                         10 * sizeof(float4) +                 // ray, shadow ray, throughput, radiance, hit, sample, ...
+                         3 * sizeof(int) +                     // eta of the sample, flags, occlusion
                          2 +                                   // splat pix_irregular
                          (3 + RT_NQUEUE) * sizeof(int) +       // end closest shadow, shading and finish queues
                          3 * sizeof(int);                      // sid, sort keys and scratch
-    return wave + (volpath ? 6 * (int64_t)sizeof(float4) : 0);   // v_seg v_p v_li0 v_li1 v_li2 v_val
+    return wave + (volpath ? 6 * (int64_t)sizeof(float4) : 0);   // v_light v_point v_val (2 each)
 }
 
 static rt_status ensure_wave(rt_ctx *c, int capacity, int max_rounds)
@@ -3166,20 +3171,11 @@ static rt_status ensure_wave(rt_ctx *c, int capacity, int max_rounds)
         return true;
     };
     bool ok = true;
-    ok &= alloc((void **)&W.rng, P * sizeof(Pcg32));
-    ok &= alloc((void **)&W.tp, P * sizeof(float4));
-    ok &= alloc((void **)&W.rad, P * sizeof(float4));
-    ok &= alloc((void **)&W.ray_o, P * sizeof(float4));
-    ok &= alloc((void **)&W.ray_d, P * sizeof(float4));
+    ok &= alloc((void **)&W.ray, 2 * P * sizeof(float4));
+    ok &= alloc((void **)&W.acc, 2 * P * sizeof(float4));
+    ok &= alloc((void **)&W.smp, 2 * P * sizeof(float4));
     ok &= alloc((void **)&W.hit, P * sizeof(float4));
-    ok &= alloc((void **)&W.bs, P * sizeof(float4));
-    ok &= alloc((void **)&W.rel_eta, P * sizeof(float));
-    ok &= alloc((void **)&W.flags, P * sizeof(int));
-    ok &= alloc((void **)&W.nee, P * sizeof(float4));
-    ok &= alloc((void **)&W.sh_o, P * sizeof(float4));
-    ok &= alloc((void **)&W.sh_d, P * sizeof(float4));
-    ok &= alloc((void **)&W.occl, P * sizeof(int));
-    ok &= alloc((void **)&W.out, P * sizeof(float4));
+    ok &= alloc((void **)&W.sh, 2 * P * sizeof(float4));
     ok &= alloc((void **)&W.splat, P);
     ok &= alloc((void **)&W.pix_irregular, P);
     ok &= alloc((void **)&W.q_end, P * sizeof(int));
@@ -4063,7 +4059,8 @@ rt_status rt_render_paths(rt_ctx *ctx, rt_scene *sc, const rt_render_desc *rd, c
                 if (nc.closest == 0 && nc.end == 0) break;
             }
         }
-        CK(cudaMemcpyAsync(out.data(), ctx->W.out, (size_t)n * sizeof(float4), cudaMemcpyDeviceToHost, st));
+        CK(cudaMemcpy2DAsync(out.data(), sizeof(float4), ctx->W.acc + 1, 2 * sizeof(float4), sizeof(float4), (size_t)n,
+                             cudaMemcpyDeviceToHost, st));
         int limit = 0;
         CK(cudaMemcpyAsync(&limit, ctx->limit_flag, sizeof(int), cudaMemcpyDeviceToHost, st));
         CK(cudaStreamSynchronize(st));
@@ -4323,20 +4320,11 @@ extern "C" rt_status rt_render_tile_static(rt_ctx *ctx, rt_scene *sc, const rt_r
     Wave W;
     std::memset(&W, 0, sizeof(W));
     const size_t P = (size_t)paths;
-    W.rng = (Pcg32 *)take(P * sizeof(Pcg32));
-    W.tp = (float4 *)take(P * sizeof(float4));
-    W.rad = (float4 *)take(P * sizeof(float4));
-    W.ray_o = (float4 *)take(P * sizeof(float4));
-    W.ray_d = (float4 *)take(P * sizeof(float4));
+    W.ray = (float4 *)take(2 * P * sizeof(float4));
+    W.acc = (float4 *)take(2 * P * sizeof(float4));
+    W.smp = (float4 *)take(2 * P * sizeof(float4));
     W.hit = (float4 *)take(P * sizeof(float4));
-    W.bs = (float4 *)take(P * sizeof(float4));
-    W.rel_eta = (float *)take(P * sizeof(float));
-    W.flags = (int *)take(P * sizeof(int));
-    W.nee = (float4 *)take(P * sizeof(float4));
-    W.sh_o = (float4 *)take(P * sizeof(float4));
-    W.sh_d = (float4 *)take(P * sizeof(float4));
-    W.occl = (int *)take(P * sizeof(int));
-    W.out = (float4 *)take(P * sizeof(float4));
+    W.sh = (float4 *)take(2 * P * sizeof(float4));
     W.splat = (uint8_t *)take(P);
     W.pix_irregular = (uint8_t *)take((size_t)npix);
     W.q_mat[RT_QUEUE_FIN] = (int *)take(P * sizeof(int));
@@ -4354,6 +4342,29 @@ extern "C" rt_status rt_render_tile_static(rt_ctx *ctx, rt_scene *sc, const rt_r
     unsigned long long *stats = (unsigned long long *)take(8 * sizeof(unsigned long long));
     int *limit_flag = (int *)take(sizeof(int));
     int *work = (int *)take(sizeof(int));
+    // The requests that fit are those that fitted when the path state was
+    // one array per field (229 bytes per path and queue entries, about 15 %
+    // more than now): the line callers plan their tiles by stays.
+    {
+        size_t fields = 0;
+        auto count = [&](size_t bytes, int n) {
+            for (int k = 0; k < n; k++) fields = ((fields + 255) & ~(size_t)255) + bytes;
+        };
+        count(P * 16, 7);                                              // stream, ray and hit, throughput
+        count(P * 4, 2);
+        count(P * 16, 3);
+        count(P * 4, 1);
+        count(P * 16, 1);
+        count(P, 1);
+        count((size_t)npix, 1);
+        count(P * 4, 4 + RT_NBSDF + (sc->S.has_mixed ? 1 : 0));        // queues
+        count((size_t)(rounds + 2) * sizeof(RoundCounters), 1);
+        count((size_t)npix * sizeof(int4), 1);
+        count((size_t)(RT_STATIC_MAX_LIGHTS + 1) * sizeof(float), 1);
+        count(8 * sizeof(unsigned long long), 1);
+        count(sizeof(int), 2);
+        off = std::max(off, fields);
+    }
     if (off > RT_STATIC_SCRATCH_BYTES) {
         char msg[256];
         snprintf(msg, sizeof(msg),

@@ -8,7 +8,7 @@
 namespace rtgpu {
 
 // path flags
-enum { F_FIRST = 1, F_DELTA = 2, F_NEE = 4, F_END = 8, F_DONE = 16 };
+enum { F_FIRST = 1, F_DELTA = 2, F_NEE = 4, F_END = 8 };
 
 #define RT_NBSDF 6        // sorted shading queues (bsdf_queue): types 0-4, then the delta types;
                           // RT_QUEUE_MIXED (rt_device.cuh) is one more: textured BSDFs, and
@@ -24,21 +24,24 @@ struct RoundCounters {   // one per wavefront round, zeroed per batch
     int pad[2];
 };
 
+// Path state.  What a kernel reads or writes together lies together, in
+// records of 32 bytes (two float4, one memory sector): the queues hold the
+// slots in the order the traversal finished them, so beyond the first bounces
+// a warp's accesses scatter, and a lone 16-byte field moves a whole sector for
+// half of it (740 bytes of DRAM per shaded vertex against about 310 used).
+// Against an array per field: furnished room (1024^2 x 16 spp) 24.3 -> 16.4 ms,
+// its shading 15.8 -> 7.9; 1.31M-triangle frame 48.3 -> 43.0 ms, shading 17.7 ->
+// 11.9; 128^3 grid-medium frame 48.0 -> 43.0 ms.  (A hit padded to a sector of
+// its own was 1-2 % slower than its 16 bytes.)
 struct Wave {
     // per path slot
-    Pcg32 *rng;
-    float4 *tp;        // throughput rgb, eta
-    float4 *rad;       // radiance rgb, depth (int bits)
-    float4 *ray_o;     // origin, mint
-    float4 *ray_d;     // direction, maxt
+    float4 *ray;       // 2: (origin, mint), (direction, maxt)
+    float4 *acc;       // 2: (throughput rgb, eta after the pending sample), (radiance rgb, depth (int bits)); the
+                       //    radiance of a path that has ended is what the film sums (w_done)
+    float4 *smp;       // 2: (pending BSDF sample value rgb, pdf), (stream state, stream increment, flags; path_rng)
     float4 *hit;       // t, u, v, prim (int bits)
-    float4 *bs;        // pending BSDF sample value rgb, pdf
-    float *rel_eta;
-    int *flags;
-    float4 *nee;       // pending light-sample contribution rgb
-    float4 *sh_o, *sh_d;
-    int *occl;
-    float4 *out;       // final radiance rgb, nan flag
+    float4 *sh;        // 2: light sample's shadow ray (direction, maxt; it starts at the ray's origin with its mint),
+                       //    (pending contribution rgb, occluded (int bits, written by the any-hit trace))
     uint8_t *splat;    // film footprint code of the sample
     uint8_t *pix_irregular;  // per batch pixel: some sample splats off its pixel
     // queues of the current round
@@ -55,14 +58,67 @@ struct Wave {
     int capacity;
     int max_rounds;
     // VolPathTracing wavefront (allocated only for it, vw_capacity paths)
-    float4 *v_seg;     // origin of the ray segment that found `hit` (its direction is the path's), medium
-    float4 *v_p;       // vertex position (scatter point or surface point), light-selection weight
-    float4 *v_li0;     // light sample: direction to the light, distance
-    float4 *v_li1;     // light sample: point on the light, pdf
-    float4 *v_li2;     // light sample: normal at the point
-    float4 *v_val;     // light sample intensity, then the attenuated light-sample value
+    float4 *v_light;   // 2: (vertex position, light-selection weight), (direction to the sampled light, distance)
+    float4 *v_point;   // 2: (point on the light, pdf), (normal at the point, delta light)
+    float4 *v_val;     // 2: (light sample intensity, then its attenuated value), (origin of the ray segment that
+                       //    found `hit` (its direction is the path's), medium)
     int vw_capacity;
 };
+__device__ __forceinline__ float4 &w_ray_o(const Wave &W, int s) { return W.ray[2 * (size_t)s]; }
+__device__ __forceinline__ float4 &w_ray_d(const Wave &W, int s) { return W.ray[2 * (size_t)s + 1]; }
+__device__ __forceinline__ float4 &w_tp(const Wave &W, int s) { return W.acc[2 * (size_t)s]; }
+__device__ __forceinline__ float4 &w_rad(const Wave &W, int s) { return W.acc[2 * (size_t)s + 1]; }
+// both halves of a slot's record in one 32-byte access
+__device__ __forceinline__ void w_load2(const float4 *rec, int s, float4 &a, float4 &b)
+{
+    const float4 *p = rec + 2 * (size_t)s;
+    asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+                 : "l"(p)
+                 : "memory");
+}
+__device__ __forceinline__ void w_store2(float4 *rec, int s, float4 a, float4 b)
+{
+    float4 *p = rec + 2 * (size_t)s;
+    asm volatile("st.global.v8.f32 [%8], {%0, %1, %2, %3, %4, %5, %6, %7};"
+                 :
+                 : "f"(a.x), "f"(a.y), "f"(a.z), "f"(a.w), "f"(b.x), "f"(b.y), "f"(b.z), "f"(b.w), "l"(p)
+                 : "memory");
+}
+// a path's end: its whole record, so that the sector need not be read for it
+__device__ __forceinline__ void w_done(const Wave &W, int s, C3 L)
+{
+    w_store2(W.acc, s, make_float4(0.f, 0.f, 0.f, 0.f), make_float4(L.r, L.g, L.b, 0.f));
+}
+__device__ __forceinline__ float4 &w_bs(const Wave &W, int s) { return W.smp[2 * (size_t)s]; }
+__device__ __forceinline__ float4 &w_rng(const Wave &W, int s) { return W.smp[2 * (size_t)s + 1]; }
+__device__ __forceinline__ float4 &w_sh_d(const Wave &W, int s) { return W.sh[2 * (size_t)s]; }
+__device__ __forceinline__ float4 &w_nee(const Wave &W, int s) { return W.sh[2 * (size_t)s + 1]; }
+__device__ __forceinline__ void w_set_occluded(const Wave &W, int s, bool o) { w_nee(W, s).w = __int_as_float(o ? 1 : 0); }
+__device__ __forceinline__ float4 &w_v_p(const Wave &W, int s) { return W.v_light[2 * (size_t)s]; }
+__device__ __forceinline__ float4 &w_v_li0(const Wave &W, int s) { return W.v_light[2 * (size_t)s + 1]; }
+__device__ __forceinline__ float4 &w_v_li1(const Wave &W, int s) { return W.v_point[2 * (size_t)s]; }
+__device__ __forceinline__ float4 &w_v_li2(const Wave &W, int s) { return W.v_point[2 * (size_t)s + 1]; }
+__device__ __forceinline__ float4 &w_v_val(const Wave &W, int s) { return W.v_val[2 * (size_t)s]; }
+__device__ __forceinline__ float4 &w_v_seg(const Wave &W, int s) { return W.v_val[2 * (size_t)s + 1]; }
+// A path's stream and flags in 16 bytes: the state, the increment's low word,
+// the flags (31 bits) with the increment's bit 32 on top (an increment is
+// twice a 32-bit sample index plus one).
+__device__ __forceinline__ float4 path_rng_pack(const Pcg32 &r, int flags)
+{
+    return make_float4(__uint_as_float((unsigned)r.state), __uint_as_float((unsigned)(r.state >> 32)),
+                       __uint_as_float((unsigned)r.inc),
+                       __uint_as_float(((unsigned)flags & 0x7fffffffu) | ((unsigned)(r.inc >> 32) << 31)));
+}
+__device__ __forceinline__ Pcg32 path_rng(float4 v, int &flags)
+{
+    const unsigned w = __float_as_uint(v.w);
+    Pcg32 r;
+    r.state = (uint64_t)__float_as_uint(v.x) | (uint64_t)__float_as_uint(v.y) << 32;
+    r.inc = (uint64_t)__float_as_uint(v.z) | (uint64_t)(w >> 31) << 32;
+    flags = (int)(w & 0x7fffffffu);
+    return r;
+}
 
 // One work item of a multi-scene batch (rt_internal_render_multi): whole
 // tiles of one job with every sample of their pixels.  The batch's path

@@ -307,8 +307,9 @@ __global__ void __launch_bounds__(128, RT_VOLPATH_MINB) k_volpath(RenderParams P
                 int q = base + __popc(need & ((1u << lane) - 1));
                 if (q < P.n_paths) {
                     slot = q;
-                    rng = P.W.rng[slot];
-                    float4 ro = P.W.ray_o[slot], rd = P.W.ray_d[slot];
+                    int flags;
+                    rng = path_rng(w_rng(P.W, slot), flags);
+                    float4 ro = w_ray_o(P.W, slot), rd = w_ray_d(P.W, slot);
                     vol_start(P.S, st, make_ray(xyz(ro), xyz(rd), ro.w, rd.w));
                     active = true;
                 } else {
@@ -318,7 +319,7 @@ __global__ void __launch_bounds__(128, RT_VOLPATH_MINB) k_volpath(RenderParams P
         }
         if (!__any_sync(0xffffffffu, active)) break;
         if (active && !vol_step(P.S, st, rng, P.max_depth, P.min_depth, limit)) {
-            P.W.out[slot] = f4c(st.L, 0.f);
+            w_done(P.W, slot, st.L);
             active = false;
         }
     }
@@ -378,13 +379,12 @@ __device__ __forceinline__ bool vw_light_pick(const DevScene &S, V3 p, Pcg32 &rn
 }
 __device__ __forceinline__ void vw_store_light(const RenderParams &P, int slot, const LightRec &li, V3 p, float lw)
 {
-    P.W.v_p[slot] = f4(p, lw);
-    P.W.v_li0[slot] = f4(li.to_light, li.distance);
-    P.W.v_li1[slot] = f4(li.point, li.pdf);
-    P.W.v_li2[slot] = f4(li.normal, li.delta ? 1.f : 0.f);
-    P.W.v_val[slot] = f4c(li.intensity, 0.f);
+    w_v_p(P.W, slot) = f4(p, lw);
+    w_v_li0(P.W, slot) = f4(li.to_light, li.distance);
+    w_v_li1(P.W, slot) = f4(li.point, li.pdf);
+    w_v_li2(P.W, slot) = f4(li.normal, li.delta ? 1.f : 0.f);
+    w_v_val(P.W, slot) = f4c(li.intensity, 0.f);
 }
-__device__ __forceinline__ void vw_done(const RenderParams &P, int slot, C3 L) { P.W.out[slot] = f4c(L, 0.f); }
 
 // evalTransmittanceFromSampledBSDF (VolPathTracing.cpp:369-424), as
 // eval_tr_sampled, reporting the segment origin of the hit instead of its
@@ -504,9 +504,11 @@ __device__ __forceinline__ unsigned vw_step_path(const RenderParams &P, const De
 {
     unsigned want = 0;
     // ---- the trace (k_vw_trace)
-    int flags = P.W.flags[slot];
-    const float4 ro = P.W.ray_o[slot], rd = P.W.ray_d[slot];
-    float4 radv = P.W.rad[slot];
+    int flags;
+    Pcg32 rng = path_rng(w_rng(P.W, slot), flags);
+    const float4 ro = w_ray_o(P.W, slot), rd = w_ray_d(P.W, slot);
+    const float4 tpv = w_tp(P.W, slot);
+    float4 radv = w_rad(P.W, slot);
     float4 seg;
     Hit h;
     const bool traces = (flags & (VF_FIRST | VF_NULLX)) != 0;
@@ -517,7 +519,7 @@ __device__ __forceinline__ unsigned vw_step_path(const RenderParams &P, const De
     } else {
         const float4 hv = P.W.hit[slot];
         h.t = hv.x; h.u = hv.y; h.v = hv.z; h.prim = __float_as_int(hv.w);
-        seg = P.W.v_seg[slot];
+        seg = w_v_seg(P.W, slot);
         if (!(flags & VF_NULLX)) {   // the trace that ends a bounce
             flags &= ~VF_EMISSION;
             radv.w = __int_as_float(__float_as_int(radv.w) + 1);
@@ -534,18 +536,16 @@ __device__ __forceinline__ unsigned vw_step_path(const RenderParams &P, const De
         P.W.hit[slot] = make_float4(h.t, h.u, h.v, __int_as_float(h.prim));
     }
     // ---- the step (k_vw_step)
-    const float4 tpv = P.W.tp[slot];
     C3 L = rgb(radv), T = rgb(tpv);
     const int depth = __float_as_int(radv.w);
     bool push_shadow = false, push_sample = false, push_trace = false;
     int guard = (flags >> VF_GUARD_SHIFT) + 1;
     if (depth >= P.max_depth) {
-        vw_done(P, slot, L);
+        w_done(P.W, slot, L);
     } else if (guard > (1 << 16)) {
         limit = 1;
-        vw_done(P, slot, L);
+        w_done(P.W, slot, L);
     } else {
-        Pcg32 rng = P.W.rng[slot];
         Ray ray = make_ray(xyz(ro), xyz(rd), ro.w, rd.w);
         int medium = __float_as_int(seg.w);
         float t = 0.f;
@@ -577,8 +577,8 @@ __device__ __forceinline__ unsigned vw_step_path(const RenderParams &P, const De
                     ray = make_ray(fr.p, ray.d, RT_EPSILON, RT_MAX_REAL);
                     if (prim_interior(S, h.prim) != prim_exterior(S, h.prim))
                         medium = dot(fr.n, ray.d) < 0.f ? prim_interior(S, h.prim) : prim_exterior(S, h.prim);
-                    P.W.ray_o[slot] = f4(ray.o, ray.mint);
-                    P.W.ray_d[slot] = f4(ray.d, ray.maxt);
+                    w_ray_o(P.W, slot) = f4(ray.o, ray.mint);
+                    w_ray_d(P.W, slot) = f4(ray.d, ray.maxt);
                     flags |= VF_NULLX;
                     push_trace = true;
                 } else {
@@ -598,13 +598,12 @@ __device__ __forceinline__ unsigned vw_step_path(const RenderParams &P, const De
             flags &= ~VF_HASVAL;
         }
         if (done) {
-            vw_done(P, slot, L);
+            w_done(P.W, slot, L);
         } else {
-            P.W.rng[slot] = rng;
-            P.W.rad[slot] = f4c(L, __int_as_float(depth));
-            P.W.tp[slot] = f4c(T, tpv.w);
-            P.W.v_seg[slot] = make_float4(seg.x, seg.y, seg.z, __int_as_float(medium));
-            P.W.flags[slot] = (flags & ((1 << VF_GUARD_SHIFT) - 1)) | (guard << VF_GUARD_SHIFT);
+            w_rad(P.W, slot) = f4c(L, __int_as_float(depth));
+            w_tp(P.W, slot) = f4c(T, tpv.w);
+            w_v_seg(P.W, slot) = make_float4(seg.x, seg.y, seg.z, __int_as_float(medium));
+            w_rng(P.W, slot) = path_rng_pack(rng, (flags & ((1 << VF_GUARD_SHIFT) - 1)) | (guard << VF_GUARD_SHIFT));
         }
     }
     want = push_shadow ? 1u : push_sample ? ((flags & VF_SCAT) ? 2u : 4u) : push_trace ? 8u : 0u;
@@ -632,17 +631,16 @@ __global__ void __launch_bounds__(128, RT_VW_MINB_STEP) k_vw_trace_step(RenderPa
 __device__ __forceinline__ unsigned vw_shadow_path(const RenderParams &P, const DevScene &S, int slot, int &limit)
 {
     unsigned want = 0;
-    Pcg32 rng = P.W.rng[slot];
-    float4 pv = P.W.v_p[slot], l0 = P.W.v_li0[slot], l1 = P.W.v_li1[slot], iv = P.W.v_val[slot];
-    const int medium = __float_as_int(P.W.v_seg[slot].w);
+    int flags;
+    Pcg32 rng = path_rng(w_rng(P.W, slot), flags);
+    float4 pv = w_v_p(P.W, slot), l0 = w_v_li0(P.W, slot), l1 = w_v_li1(P.W, slot), iv = w_v_val(P.W, slot);
+    const int medium = __float_as_int(w_v_seg(P.W, slot).w);
     C3 tr = vw_transmittance(S, make_ray(xyz(pv), xyz(l0), RT_EPSILON, l0.w - RT_EPSILON), medium, rng, limit);
     float pdf = l1.w * pv.w;
     C3 value = (tr * rgb(iv)) / pdf;
-    P.W.v_li1[slot] = make_float4(l1.x, l1.y, l1.z, pdf);
-    P.W.v_val[slot] = f4c(value, 0.f);
-    P.W.rng[slot] = rng;
-    const int flags = P.W.flags[slot] | VF_HASVAL;
-    P.W.flags[slot] = flags;
+    w_v_li1(P.W, slot) = make_float4(l1.x, l1.y, l1.z, pdf);
+    w_v_val(P.W, slot) = f4c(value, 0.f);
+    w_rng(P.W, slot) = path_rng_pack(rng, flags | VF_HASVAL);
     want = (flags & VF_SCAT) ? 1u : 2u;
     return want;
 }
@@ -670,16 +668,16 @@ __global__ void __launch_bounds__(128, RT_VW_MINB_SHADOW) k_vw_shadow(RenderPara
 __device__ __forceinline__ unsigned vw_surface_path(const RenderParams &P, const DevScene &S, int slot)
 {
     unsigned want = 0;
-    int flags = P.W.flags[slot];
-    Pcg32 rng = P.W.rng[slot];
-    float4 radv = P.W.rad[slot], tpv = P.W.tp[slot];
+    int flags;
+    Pcg32 rng = path_rng(w_rng(P.W, slot), flags);
+    float4 radv = w_rad(P.W, slot), tpv = w_tp(P.W, slot);
     C3 L = rgb(radv), T = rgb(tpv);
-    float4 ro = P.W.ray_o[slot], rd = P.W.ray_d[slot];
+    float4 ro = w_ray_o(P.W, slot), rd = w_ray_d(P.W, slot);
     Ray ray = make_ray(xyz(ro), xyz(rd), ro.w, rd.w);
-    float4 seg = P.W.v_seg[slot];
+    float4 seg = w_v_seg(P.W, slot);
     int medium = __float_as_int(seg.w);
     const bool hasval = flags & VF_HASVAL;
-    C3 value = hasval ? rgb(P.W.v_val[slot]) : cfill(0.f);
+    C3 value = hasval ? rgb(w_v_val(P.W, slot)) : cfill(0.f);
     bool push = true;
     {
         float4 hv = P.W.hit[slot];
@@ -694,11 +692,11 @@ __device__ __forceinline__ unsigned vw_surface_path(const RenderParams &P, const
         }
         const DevBsdf &B = *Bp;
         if (!iszero(value)) {
-            V3 to_light = xyz(P.W.v_li0[slot]);
-            float lpdf = P.W.v_li1[slot].w;
+            V3 to_light = xyz(w_v_li0(P.W, slot));
+            float lpdf = w_v_li1(P.W, slot).w;
             V3 wi = to_local(fr, to_light), wo = to_local(fr, -ray.d);
             float ct = fabsf(wi.z);
-            float bp = P.W.v_li2[slot].w != 0.f ? 0.f : any_bsdf_pdf(B, wi, wo);
+            float bp = w_v_li2(P.W, slot).w != 0.f ? 0.f : any_bsdf_pdf(B, wi, wo);
             float w = power_heuristic(lpdf, bp);
             L = L + (((T * value) * any_bsdf_eval(B, wi, wo)) * ct) * w;
         }
@@ -708,24 +706,24 @@ __device__ __forceinline__ unsigned vw_surface_path(const RenderParams &P, const
         V2 bu = next2d(rng);
         C3 f = any_bsdf_sample(B, r, bu, rng.state);
         if (iszero(f)) {
-            vw_done(P, slot, L);
+            w_done(P.W, slot, L);
             push = false;
         } else {
             ray = make_ray(fr.p, to_world(fr, r.wo), RT_EPSILON, RT_MAX_REAL);
             if (prim_interior(S, h.prim) != prim_exterior(S, h.prim))
                 medium = dot(fr.n, ray.d) < 0.f ? prim_interior(S, h.prim) : prim_exterior(S, h.prim);
-            P.W.bs[slot] = f4c(f, r.pdf);
-            P.W.rel_eta[slot] = r.rel_eta;
+            w_bs(P.W, slot) = f4c(f, r.pdf);
+            tpv.w *= r.rel_eta;   // eta as the end of the pass reads it
             flags = (r.type & BT_DELTA) ? (flags | VF_DELTA) : (flags & ~VF_DELTA);
         }
     }
     if (push) {
-        P.W.rng[slot] = rng;
-        P.W.rad[slot] = f4c(L, radv.w);
-        P.W.ray_o[slot] = f4(ray.o, ray.mint);
-        P.W.ray_d[slot] = f4(ray.d, ray.maxt);
-        P.W.v_seg[slot] = make_float4(seg.x, seg.y, seg.z, __int_as_float(medium));
-        P.W.flags[slot] = flags;
+        w_tp(P.W, slot) = tpv;
+        w_rad(P.W, slot) = f4c(L, radv.w);
+        w_ray_o(P.W, slot) = f4(ray.o, ray.mint);
+        w_ray_d(P.W, slot) = f4(ray.d, ray.maxt);
+        w_v_seg(P.W, slot) = make_float4(seg.x, seg.y, seg.z, __int_as_float(medium));
+        w_rng(P.W, slot) = path_rng_pack(rng, flags);
     }
     want = push ? 1u : 0u;
     return want;
@@ -769,8 +767,8 @@ __device__ __forceinline__ bool vw_finish_one(const RenderParams &P, const DevSc
             if (hl >= 0) {
                 Frame fr = hit_frame(S, h, xyz(seg), d);
                 C3 Le = area_le(S, hl, -d, fr.n);
-                float pl = light_pdf(S, hl, fr.p, xyz(P.W.v_li1[slot]), xyz(P.W.v_li2[slot]),
-                                        xyz(P.W.v_li0[slot]));
+                float pl = light_pdf(S, hl, fr.p, xyz(w_v_li1(P.W, slot)), xyz(w_v_li2(P.W, slot)),
+                                        xyz(w_v_li0(P.W, slot)));
                 float w = power_heuristic(bsv.w, pl);
                 L = L + ((T * Le) * tr) * w;
             }
@@ -794,15 +792,12 @@ __device__ __forceinline__ bool vw_finish_one(const RenderParams &P, const DevSc
             if (S.env_light >= 0) { caught = S.env_light; isenv = true; Le = env_le(S.lights[S.env_light], d); }
         }
         if (caught >= 0) {
-            float pl = (flags & VF_DELTA) ? 0.f : light_pdf(S, caught, xyz(P.W.v_p[slot]), fr.p, fr.n, d);
+            float pl = (flags & VF_DELTA) ? 0.f : light_pdf(S, caught, xyz(w_v_p(P.W, slot)), fr.p, fr.n, d);
             float w = power_heuristic(bsv.w, pl);
             L = L + (((T * Le) * f) * tr) * w;
             if (isenv && medium < 0) done = true;
         }
-        if (!done) {
-            T = T * f;
-            eta *= P.W.rel_eta[slot];
-        }
+        if (!done) T = T * f;
     }
     if (!done && depth >= P.min_depth) {
         float stop = smin(0.95f, cmax(T) * eta * eta);
@@ -810,16 +805,15 @@ __device__ __forceinline__ bool vw_finish_one(const RenderParams &P, const DevSc
         else done = true;
     }
     if (done) {
-        vw_done(P, slot, L);
+        w_done(P.W, slot, L);
     } else {
-        P.W.rng[slot] = rng;
-        P.W.ray_o[slot] = ro;
-        P.W.ray_d[slot] = rd;
+        w_ray_o(P.W, slot) = ro;
+        w_ray_d(P.W, slot) = rd;
         P.W.hit[slot] = make_float4(h1.t, h1.u, h1.v, __int_as_float(h1.prim));
-        P.W.v_seg[slot] = seg1;
-        P.W.flags[slot] = (flags & ~VF_WAS) | (was1 ? VF_WAS : 0);
-        P.W.rad[slot] = f4c(L, __int_as_float(depth));
-        P.W.tp[slot] = f4c(T, eta);
+        w_v_seg(P.W, slot) = seg1;
+        w_rng(P.W, slot) = path_rng_pack(rng, (flags & ~VF_WAS) | (was1 ? VF_WAS : 0));
+        w_rad(P.W, slot) = f4c(L, __int_as_float(depth));
+        w_tp(P.W, slot) = f4c(T, eta);
     }
     return !done;
 }
@@ -829,12 +823,12 @@ __device__ __forceinline__ bool vw_finish_one(const RenderParams &P, const DevSc
 __device__ __forceinline__ unsigned vw_trsamp_path(const RenderParams &P, const DevScene &S, int slot, int &limit)
 {
     unsigned want = 0;
-    int flags = P.W.flags[slot];
-    Pcg32 rng = P.W.rng[slot];
-    const float4 ro = P.W.ray_o[slot], rd = P.W.ray_d[slot];
+    int flags;
+    Pcg32 rng = path_rng(w_rng(P.W, slot), flags);
+    const float4 ro = w_ray_o(P.W, slot), rd = w_ray_d(P.W, slot);
     const float4 hv = P.W.hit[slot];
     Hit h; h.t = hv.x; h.u = hv.y; h.v = hv.z; h.prim = __float_as_int(hv.w);
-    float4 seg = P.W.v_seg[slot];
+    float4 seg = w_v_seg(P.W, slot);
     V3 so = xyz(seg);
     Hit h1;
     bool was, was1;
@@ -844,9 +838,9 @@ __device__ __forceinline__ unsigned vw_trsamp_path(const RenderParams &P, const 
     flags = (flags & ~VF_NEWM) | (newm >= 0 ? VF_NEWM : 0);
     const float4 seg1 = was1 ? make_float4(ro.x, ro.y, ro.z, seg.w) : seg;
     seg = make_float4(so.x, so.y, so.z, seg.w);
-    const float4 radv = P.W.rad[slot];
+    const float4 radv = w_rad(P.W, slot);
     want = vw_finish_one<false>(P, S, slot, flags, rng, ro, rd, seg, h, was, h1, was1, seg1, tr, rgb(radv), __float_as_int(radv.w),
-                         P.W.tp[slot], P.W.bs[slot])
+                         w_tp(P.W, slot), w_bs(P.W, slot))
                ? 1u
                : 0u;
     return want;
@@ -878,15 +872,15 @@ __global__ void __launch_bounds__(128, RT_VW_MINB_TRSAMP) k_vw_trsamp_finish(Ren
 __device__ __forceinline__ unsigned vw_scatter_path(const RenderParams &P, const DevScene &S, int slot, int &limit)
 {
     unsigned want = 0;
-    int flags = P.W.flags[slot];
-    Pcg32 rng = P.W.rng[slot];
-    float4 seg = P.W.v_seg[slot];
+    int flags;
+    Pcg32 rng = path_rng(w_rng(P.W, slot), flags);
+    float4 seg = w_v_seg(P.W, slot);
     const int medium = __float_as_int(seg.w);
-    float4 rd = P.W.ray_d[slot];
+    float4 rd = w_ray_d(P.W, slot);
     V3 wo;
     float pfpdf;
     const float pfw = phase_sample(S.media[medium], -xyz(rd), next2d(rng), wo, pfpdf);
-    const float4 ro = f4(xyz(P.W.v_p[slot]), 0.f);
+    const float4 ro = f4(xyz(w_v_p(P.W, slot)), 0.f);
     rd = f4(wo, rd.w);
     const float4 hv = P.W.hit[slot];
     Hit h; h.t = hv.x; h.u = hv.y; h.v = hv.z; h.prim = __float_as_int(hv.w);
@@ -899,16 +893,16 @@ __device__ __forceinline__ unsigned vw_scatter_path(const RenderParams &P, const
     const float4 seg1 = was1 ? make_float4(ro.x, ro.y, ro.z, seg.w) : seg;
     seg = make_float4(so.x, so.y, so.z, seg.w);
     // the light sample's MIS at the scatter point
-    const float4 radv = P.W.rad[slot], tpv = P.W.tp[slot];
+    const float4 radv = w_rad(P.W, slot), tpv = w_tp(P.W, slot);
     C3 L = rgb(radv);
     if (flags & VF_HASVAL) {
-        const C3 value = rgb(P.W.v_val[slot]);
+        const C3 value = rgb(w_v_val(P.W, slot));
         if (!iszero(value)) {
             const DevMedium &M = S.media[medium];
-            const V3 din = xyz(P.W.ray_d[slot]);
-            const V3 to_light = xyz(P.W.v_li0[slot]);
-            const float lpdf = P.W.v_li1[slot].w;
-            const float pf = P.W.v_li2[slot].w != 0.f ? 0.f : phase_eval(M, to_light, -din);
+            const V3 din = xyz(w_ray_d(P.W, slot));
+            const V3 to_light = xyz(w_v_li0(P.W, slot));
+            const float lpdf = w_v_li1(P.W, slot).w;
+            const float pf = w_v_li2(P.W, slot).w != 0.f ? 0.f : phase_eval(M, to_light, -din);
             const float w = power_heuristic(lpdf, pf);
             const float ev = phase_eval(M, to_light, -din);
             L = L + ((rgb(tpv) * value) * ev) * w;
