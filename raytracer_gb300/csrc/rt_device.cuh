@@ -57,7 +57,9 @@ struct DevTexture {
 
 // Shading queue of a BSDF.  The heavy types (0-4) get a queue and a shading
 // kernel each; the smooth (delta) types Dielectric, Conductor and Mirror
-// (5-7) are cheap and share one; textured BSDFs of any type go to the mixed
+// (5-7) are cheap and share one.  Textured BSDFs go to their type's queue,
+// shaded by a kernel that applies the textures, in single-scene renders with
+// one light per vertex (RenderParams::tex_types); elsewhere to the mixed
 // queue, whose kernel dispatches at run time and applies the textures.
 #define RT_QUEUE_DELTA 5
 #define RT_QUEUE_MIXED 6
@@ -66,6 +68,13 @@ __host__ __device__ __forceinline__ int bsdf_queue(int type) { return type < RT_
 __host__ __device__ __forceinline__ int bsdf_queue_of(const DevBsdf &b)
 {
     return (b.textured || b.type == 9) ? RT_QUEUE_MIXED : bsdf_queue(b.type);
+}
+// a primitive's queue code: the queue of its BSDF's type, with RT_TEXTURED
+// when the BSDF is textured
+#define RT_TEXTURED 8
+__host__ __device__ __forceinline__ int bsdf_code_of(const DevBsdf &b)
+{
+    return b.type == 9 ? RT_QUEUE_MIXED : bsdf_queue(b.type) | (b.textured ? RT_TEXTURED : 0);
 }
 
 struct DevLight {
@@ -139,7 +148,7 @@ struct DevScene {
     // 1.31M-triangle frame 0.4 % faster).
     const float4 *tri_rec;
     const float *tri_n;         // 9 floats per triangle (n0, n1, n2) or null
-    const uint8_t *tri_type;    // shading queue (bsdf_queue_of) of the triangle's mesh BSDF, 255 = no BSDF
+    const uint8_t *tri_type;    // queue code (bsdf_code_of) of the triangle's mesh BSDF, 255 = no BSDF
     const float *tri_uv;        // 6 floats per triangle (uv0, uv1, uv2) or null; NaN: mesh without uvs
     const DevTexture *textures;
     int n_textures;
@@ -514,7 +523,7 @@ __device__ __forceinline__ int prim_light(const DevScene &S, int prim)
 {
     return prim >= 0 ? __float_as_int(__ldg(&S.tri_rec[3 * (size_t)prim + 1].w)) : S.spheres[-prim - 2].light;
 }
-// shading queue (bsdf_queue) of a hit primitive's BSDF, or -1 without a BSDF
+// queue code (bsdf_code_of) of a hit primitive's BSDF, or -1 without a BSDF
 __device__ __forceinline__ int prim_type(const DevScene &S, int prim)
 {
     if (prim >= 0) {
@@ -522,7 +531,7 @@ __device__ __forceinline__ int prim_type(const DevScene &S, int prim)
         return t == 255 ? -1 : t;
     }
     int b = S.spheres[-prim - 2].bsdf;
-    return b < 0 ? -1 : bsdf_queue_of(S.bsdfs[b]);
+    return b < 0 ? -1 : bsdf_code_of(S.bsdfs[b]);
 }
 
 __device__ __forceinline__ int prim_interior(const DevScene &S, int prim)
@@ -677,7 +686,7 @@ __device__ __noinline__ C3 tex_eval(const DevTexture &T, V2 uv)
 // The BSDF parameters at a hit: textured ones replaced by their texture's
 // value at uv (an alpha texture by the average of its channels, as the
 // rough BSDFs read it).
-__device__ __noinline__ void tex_apply(const DevScene &S, DevBsdf &b, V2 uv)
+__device__ __forceinline__ void tex_apply_inline(const DevScene &S, DevBsdf &b, V2 uv)
 {
     if (b.tex[TEX_ALBEDO] >= 0) {
         C3 c = tex_eval(S.textures[b.tex[TEX_ALBEDO]], uv);
@@ -697,6 +706,7 @@ __device__ __noinline__ void tex_apply(const DevScene &S, DevBsdf &b, V2 uv)
         b.alpha_avg = a;
     }
 }
+__device__ __noinline__ void tex_apply(const DevScene &S, DevBsdf &b, V2 uv) { tex_apply_inline(S, b, uv); }
 __device__ __forceinline__ V3 cartesian_from_spherical(float theta, float phi)
 {
     float st = sinf(theta), ct = cosf(theta), cp = cosf(phi), sp = sinf(phi);
