@@ -208,10 +208,8 @@ __global__ void k_camera(RenderParams P)
             P.W.splat[slot] = code;
             if (code != 0x55) P.W.pix_irregular[q] = 1;
         }
-        const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
         w_store2(P.W.ray, slot, f4(r.o, r.mint), f4(r.d, r.maxt));
-        w_store2(P.W.acc, slot, make_float4(1.f, 1.f, 1.f, 1.f), zero);
-        w_store2(P.W.smp, slot, zero, path_rng_pack(rng, F_FIRST));
+        w_store2(P.W.smp, slot, make_float4(0.f, 0.f, 0.f, 0.f), path_rng_pack(rng, F_FIRST));
         P.W.q_closest[slot] = slot;
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -274,10 +272,8 @@ __global__ void k_camera_multi(RenderParams P)
         P.W.splat[slot] = code;
         if (code != 0x55) P.W.pix_irregular[it.pix0 + q] = 1;
         P.W.sid[slot] = it.job;
-        const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
         w_store2(P.W.ray, slot, f4(r.o, r.mint), f4(r.d, r.maxt));
-        w_store2(P.W.acc, slot, make_float4(1.f, 1.f, 1.f, 1.f), zero);
-        w_store2(P.W.smp, slot, zero, path_rng_pack(rng, F_FIRST));
+        w_store2(P.W.smp, slot, make_float4(0.f, 0.f, 0.f, 0.f), path_rng_pack(rng, F_FIRST));
         P.W.q_closest[slot] = slot;
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -1056,7 +1052,8 @@ __device__ __forceinline__ void pt_finish_path(const RenderParams &P, const DevS
 {
     const int env = S.env_light;
     const int flags = (int)(__float_as_uint(w_rng(P.W, slot).w) & 0x7fffffffu);
-    C3 L = rgb(w_rad(P.W, slot));
+    C3 L = cfill(0.f);
+    if (!(flags & F_FIRST)) L = rgb(w_rad(P.W, slot));
     if (flags & F_FIRST) {
         // camera ray: the environment if it missed; a surface without a
         // BSDF ends the path (PathTracingMIS.cpp:60-70)
@@ -1218,14 +1215,15 @@ __device__ __noinline__ C3 pt_all_lights(const DevScene &S, const DevBsdf &B, co
 }
 
 template <int BT, bool ALL = false, bool TEX = BT == RT_QUEUE_MIXED>
-__device__ __forceinline__ void pt_shade_path(const RenderParams &P, const DevScene &S, int slot, bool &push_end,
-                                              bool &push_closest, bool &push_shadow)
+__device__ __forceinline__ void pt_shade_path(const RenderParams &P, const DevScene &S, int slot, bool first_round,
+                                              bool &push_end, bool &push_closest, bool &push_shadow)
 {
     const float4 hv = P.W.hit[slot];
-    float4 ro, rd, bsv, rv, tpv, radv;
+    float4 ro, rd, bsv, rv;
     w_load2(P.W.ray, slot, ro, rd);
     w_load2(P.W.smp, slot, bsv, rv);
-    w_load2(P.W.acc, slot, tpv, radv);
+    float4 tpv = make_float4(1.f, 1.f, 1.f, 1.f), radv = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (!first_round) w_load2(P.W.acc, slot, tpv, radv);
     int flags;
     Pcg32 rng = path_rng(rv, flags);
     C3 T = rgb(tpv);
@@ -1376,8 +1374,9 @@ __global__ void __launch_bounds__(128, RT_SHADE_MINB) k_pt_shade(RenderParams P,
         int slot = valid ? qin[idx] : 0;
         bool push_end = false, push_closest = false, push_shadow = false;
         if (valid) {
-            if (MULTI) pt_shade_path<BT, ALL, TEX>(P, P.scenes[P.W.sid[slot]], slot, push_end, push_closest, push_shadow);
-            else pt_shade_path<BT, ALL, TEX>(P, P.S, slot, push_end, push_closest, push_shadow);
+            if (MULTI)
+                pt_shade_path<BT, ALL, TEX>(P, P.scenes[P.W.sid[slot]], slot, round == 0, push_end, push_closest, push_shadow);
+            else pt_shade_path<BT, ALL, TEX>(P, P.S, slot, round == 0, push_end, push_closest, push_shadow);
         }
         q_push(out_q, out_n, slot, (push_closest ? 1u : 0u) | (push_shadow ? 2u : 0u) | (push_end ? 4u : 0u));
     }
@@ -1470,7 +1469,7 @@ __global__ void __launch_bounds__(128, RT_PT_TAIL_MINB) k_pt_tail(RenderParams P
                 break;
             }
             bool push_end = false, push_closest = false, push_shadow = false;
-            pt_shade_path<RT_QUEUE_MIXED, ALL>(P, S, slot, push_end, push_closest, push_shadow);
+            pt_shade_path<RT_QUEUE_MIXED, ALL>(P, S, slot, (flags & F_FIRST) != 0, push_end, push_closest, push_shadow);
             if (!push_closest && !push_end) break;
         }
     }

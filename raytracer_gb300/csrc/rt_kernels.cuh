@@ -37,7 +37,8 @@ struct Wave {
     // per path slot
     float4 *ray;       // 2: (origin, mint), (direction, maxt)
     float4 *acc;       // 2: (throughput rgb, eta after the pending sample), (radiance rgb, depth (int bits)); the
-                       //    radiance of a path that has ended is what the film sums (w_done)
+                       //    radiance of a path that has ended is what the film sums (w_done).  Not written for a
+                       //    camera ray (F_FIRST): throughput 1, eta 1, radiance 0, depth 0
     float4 *smp;       // 2: (pending BSDF sample value rgb, pdf), (stream state, stream increment, flags; path_rng)
     float4 *hit;       // t, u, v, prim (int bits)
     float4 *sh;        // 2: light sample's shadow ray (direction, maxt; it starts at the ray's origin with its mint),

@@ -507,8 +507,8 @@ __device__ __forceinline__ unsigned vw_step_path(const RenderParams &P, const De
     int flags;
     Pcg32 rng = path_rng(w_rng(P.W, slot), flags);
     const float4 ro = w_ray_o(P.W, slot), rd = w_ray_d(P.W, slot);
-    const float4 tpv = w_tp(P.W, slot);
-    float4 radv = w_rad(P.W, slot);
+    float4 tpv = make_float4(1.f, 1.f, 1.f, 1.f), radv = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (!(flags & VF_FIRST)) w_load2(P.W.acc, slot, tpv, radv);
     float4 seg;
     Hit h;
     const bool traces = (flags & (VF_FIRST | VF_NULLX)) != 0;
