@@ -424,8 +424,16 @@ __global__ void k_sort_copy(RenderParams P, int round, int shadow)
 #define RT_FETCH_THRESHOLD 28
 #endif
 
+// resident blocks per SM: closest-hit rays carry more state, and at 10 blocks
+// (48 registers) their node loop reloads spilled values (15M local loads
+// against 4M node visits on one bounce).  9 against 10: 1.31M-triangle frame
+// 19.7 against 20.2 ms of closest hits, furnished room 5.96 / 6.20, Cornell
+// 0.44 / 0.46; any-hit rays 9.5 / 9.3 (8 is slower for both)
 #ifndef RT_TRACE_MINB
-#define RT_TRACE_MINB 10
+#define RT_TRACE_MINB 9
+#endif
+#ifndef RT_TRACE_MINB_ANY
+#define RT_TRACE_MINB_ANY 10
 #endif
 #ifndef RT_TRACE_SSTACK
 #define RT_TRACE_SSTACK 0
@@ -443,7 +451,7 @@ __global__ void k_sort_copy(RenderParams P, int round, int shadow)
 // MULTI: a multi-scene batch; each ray traverses the tree of its path's
 // scene (P.scenes[W.sid[slot]]), held per lane
 template <bool ANY, bool COUNT, bool MULTI = false>
-__global__ void __launch_bounds__(128, RT_TRACE_MINB) k_trace(RenderParams P, int round)
+__global__ void __launch_bounds__(128, ANY ? RT_TRACE_MINB_ANY : RT_TRACE_MINB) k_trace(RenderParams P, int round)
 {
     round = cur_round(P, round);
     const DevScene S = P.S;
