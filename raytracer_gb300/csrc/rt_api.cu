@@ -1207,10 +1207,11 @@ __device__ __forceinline__ C3 bsdf_sample_t(const DevBsdf &b, BsdfRec &r, V2 s, 
 // one sample of every light in turn, each with its own shadow ray (traced
 // here, any hit through the binary tree and the analytic shapes, as
 // Integrator::sampleOneLight does) and its MIS weight against the BSDF,
-// added to L in light order.  Out of line so that the shading kernels'
-// registers on the one-light path stay as they are.
+// added to L in light order.  Inline in kernels of its own (three lights,
+// 333x257 x 32 spp: 3.69 ms out of line, 3.26 inline at 8 blocks per SM, 3.4 to
+// 4.0 at 4, 5, 6, 9, 10 or 12).
 template <int BT>
-__device__ __noinline__ C3 pt_all_lights(const DevScene &S, const DevBsdf &B, const Frame &fr, V3 d, C3 T, C3 L,
+__device__ __forceinline__ C3 pt_all_lights(const DevScene &S, const DevBsdf &B, const Frame &fr, V3 d, C3 T, C3 L,
                                          Pcg32 &rng)
 {
     for (int l = 0; l < S.n_lights; l++) {
