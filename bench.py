@@ -160,7 +160,7 @@ def _config(data):
             "filter": getattr(_ARGS, "filter", "box"),
             "parallelism": "replicas" if int(os.environ.get("WORLD_SIZE", "1")) > 1 else "single",
             "l2": "inputs larger than L2: the scene (BVH, triangles, materials, maps) and the wavefront path "
-                  "state (246 bytes per path in flight, 342 for VolPathTracing) live in HBM"}
+                  "state (218 bytes per path in flight, 314 for VolPathTracing) live in HBM"}
 
 
 _ARGS = None

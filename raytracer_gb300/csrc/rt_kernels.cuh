@@ -11,8 +11,8 @@ namespace rtgpu {
 enum { F_FIRST = 1, F_DELTA = 2, F_NEE = 4, F_END = 8 };
 
 #define RT_NBSDF 6        // sorted shading queues (bsdf_queue): types 0-4, then the delta types;
-                          // RT_QUEUE_MIXED (rt_device.cuh) is one more: textured BSDFs, and
-                          // every BSDF in bounces below the sort threshold
+                          // RT_QUEUE_MIXED (rt_device.cuh) is one more: Microfacet, textured BSDFs
+                          // where they are not sorted, every BSDF in bounces below the sort threshold
 #define RT_QUEUE_FIN 7    // paths whose traced ray missed or hit a surface without a BSDF
 #define RT_NQUEUE 8
 

@@ -331,9 +331,10 @@ __global__ void __launch_bounds__(128, RT_VOLPATH_MINB) k_volpath(RenderParams P
 // over a queue of paths in HBM.  One round runs one vol_step of every live
 // path (a bounce, or a null-boundary crossing, which the reference also
 // runs as one pass of its loop):
-//   k_vw_trace_step [trace queue]  closest hit of the path's ray (the trace
-//                                  that ends vol_step / vol_start / a null
-//                                  crossing), then depth and guard, delta
+//   k_vw_trace_step [trace queue]  closest hit of a camera ray or a ray behind
+//                                  a null boundary (vol_step's last trace is
+//                                  kept from the sampled ray's first segment),
+//                                  then depth and guard, delta
 //                                  tracking through the medium, then either
 //                                  the scatter point or the surface
 //                                  (emission, null boundary, env miss), and

@@ -5,6 +5,7 @@ they are equal bit for bit, and so are the ray counts."""
 import numpy as np
 import pytest
 
+import oracle_lib as O
 from raytracer_gb300 import desc as D
 from raytracer_gb300 import scenes
 
@@ -102,3 +103,51 @@ def test_tail_batch_equals_rounds(ctx, rtlib):
             g.close()
     for a, b in zip(got, ref):
         assert np.array_equal(a, b)
+
+
+ROUNDS = {   # small films whose every path the tail kernels would take
+    "smooth": (lambda: scenes.cornell_smooth(40, 33), 4, 0.03),
+    "textured": (lambda: scenes.textured_room(41, 30), 4, 0.03),
+    "icosphere": (lambda: scenes.displaced_icosphere(level=4, width=40, height=30, env_size=(64, 32), max_depth=8), 4, 0.03),
+    "all_lights": (_delta_all, 3, 0.03),
+    "volume": (lambda: scenes.volume_grid(32, 30, res=16), 4, 0.03),
+}
+
+
+@pytest.mark.parametrize("case", sorted(ROUNDS))
+def test_rounds_match_oracle(ctx, rtlib, case):
+    """The wavefront's own rounds on small films (profiling level 2: no tail
+    kernels) against the oracle: weights bitwise, colours as the film parity
+    tests have them (a few paths flip a branch on a last-ulp difference)."""
+    make, spp, max_bad = ROUNDS[case]
+    s = make()
+    g = rtlib.Scene(ctx, s)
+    ctx.set_profiling(2)
+    try:
+        film = g.render(spp, seed=19, block=16)
+    finally:
+        ctx.set_profiling(0)
+        g.close()
+    ref = O.OracleScene(s).render(spp, seed=19, block=16)
+    assert np.array_equal(film[..., 3], ref[..., 3])
+    err = np.abs(film[..., :3] - ref[..., :3]) / np.maximum(np.abs(ref[..., :3]), 1e-3)
+    assert np.mean(err.max(-1) > 1e-3) <= max_bad
+
+
+@pytest.mark.parametrize("make", [lambda: scenes.textured_room(48, 40), lambda: scenes.plane_room(48, 40, textured=True)],
+                         ids=["textured_room", "plane_room"])
+def test_textured_queues_equal_mixed(ctx, rtlib, make):
+    """Textured BSDFs shaded from their type's queue give the film of the
+    mixed queue's run-time dispatch (a sort threshold above every round)."""
+    g = rtlib.Scene(ctx, make())
+    before = ctx.get_tuning()
+    ctx.set_profiling(2)
+    try:
+        film = g.render(5, seed=23)
+        ctx.set_tuning(sort_threshold=1 << 30)
+        mixed = g.render(5, seed=23)
+    finally:
+        ctx.set_tuning(**before)
+        ctx.set_profiling(0)
+        g.close()
+    assert np.array_equal(film, mixed)
