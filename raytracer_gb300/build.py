@@ -57,7 +57,9 @@ def build(force=False, verbose=False, ptxas_info=False):
         obj = os.path.join(BUILD, s + ".o")
         objs.append(obj)
         if force or _stale(obj, [src] + hdrs):
-            cmd = [NVCC, ARCH, "-O3", "-lineinfo", "-std=c++17", "-fmad=false", "-Xcompiler", "-fPIC",
+            # -split-compile=0: the kernels are optimised in parallel (one translation
+            # unit: 178 s one after another, 59 s on eight cores)
+            cmd = [NVCC, ARCH, "-O3", "-lineinfo", "-std=c++17", "-fmad=false", "-split-compile=0", "-Xcompiler", "-fPIC",
                    "-Xcompiler", "-ffp-contract=off",
                    "-I", os.path.join(ROOT, "include"), "-c", src, "-o", obj]
             if ptxas_info:
