@@ -8,8 +8,10 @@
 //       k_trace<any>     light-sample shadow rays         (Integrator.cpp:228-232)
 //       k_pt_shade       resolve the previous vertex, shade the new one
 //                        (PathTracingMIS.cpp:54-259), compact survivors
-//     or, for VolPathTracing, k_volpath: one persistent kernel that takes
-//     paths from a work counter and runs VolPathTracing::li to completion
+//       (a round with few paths left: k_pt_tail runs them to their end)
+//     or, for VolPathTracing, the k_vw_* rounds (rt_volpath.cuh), or k_volpath:
+//     one persistent kernel that takes paths from a work counter and runs
+//     VolPathTracing::li to completion
 //     k_film            per-pixel reduction in the reference's sample order
 //                       (Screen::addSample with the box filter, Screen::merge)
 #include "rt_kernels.cuh"
