@@ -1769,18 +1769,19 @@ __global__ void __launch_bounds__(128) k_film_wide(RenderParams P, float4 *film,
 // rt_scene_refit: new vertex positions into the triangle arrays, then the
 // binary tree's boxes bottom-up over its unchanged topology, widened as the
 // host build widens them, then the 4-wide tree's copies of them.
-__global__ void k_refit_tris(const float *vtx, const float *nrm, const int32_t *idx, int nt, float4 *tri_rec, float *tri_n)
+__global__ void k_refit_tris(const float *vtx, const float *nrm, const int32_t *idx, int nt, float *tri_rec, float *tri_n)
 {
     for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < nt; t += gridDim.x * blockDim.x)
         for (int k = 0; k < 3; k++) {
             const size_t v = (size_t)idx[3 * (size_t)t + k];
-            float4 &R = tri_rec[3 * (size_t)t + k];
-            R = make_float4(vtx[3 * v], vtx[3 * v + 1], vtx[3 * v + 2], R.w);
-            for (int a = 0; a < 3 && tri_n; a++) tri_n[9 * (size_t)t + 3 * k + a] = nrm[3 * v + a];
+            for (int a = 0; a < 3; a++) {
+                tri_rec[RT_TRI_REC * (size_t)t + 3 * k + a] = vtx[3 * v + a];
+                if (tri_n) tri_n[9 * (size_t)t + 3 * k + a] = nrm[3 * v + a];
+            }
         }
 }
 // triangle slots (p0 and id, e1 = p1 - p0, e2 = p2 - p0) from the new vertices
-__global__ void k_refit_slots(float4 *slots, int n_slots, const float4 *tri_rec)
+__global__ void k_refit_slots(float4 *slots, int n_slots, const float *tri_rec)
 {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n_slots; i += gridDim.x * blockDim.x) {
         const float4 a = slots[3 * (size_t)i];
@@ -1794,7 +1795,7 @@ __global__ void k_refit_slots(float4 *slots, int n_slots, const float4 *tri_rec)
 // one level of internal nodes: the exact boxes of both children (a leaf's
 // triangles, or an internal child's two boxes from the deeper level) into
 // boxes[12 * node]: child 0 then child 1, each (min xyz, max xyz)
-__global__ void k_refit_level(const float4 *nodes, const float4 *slots, const float4 *tri_rec, const int32_t *order,
+__global__ void k_refit_level(const float4 *nodes, const float4 *slots, const float *tri_rec, const int32_t *order,
                               int begin, int end, float *boxes)
 {
     for (int i = begin + blockIdx.x * blockDim.x + threadIdx.x; i < end; i += gridDim.x * blockDim.x) {
@@ -2861,13 +2862,14 @@ static rt_status scene_create(rt_ctx *ctx, const rt_scene_desc *d, const ExtTree
             D.env_radius = 2 * h_smax(norm(bmn - c), norm(bmx - c));
             const float *dp;
             std::vector<float4> texels((size_t)Wd * H);
-            for (size_t i = 0; i < texels.size(); i++)
-                texels[i] = make_float4(L.env_rgb[3 * i], L.env_rgb[3 * i + 1], L.env_rgb[3 * i + 2], 0.f);
+            for (int i = 0; i < H; i++)
+                for (int j = 0; j < Wd; j++) {
+                    const float *p = L.env_rgb + 3 * ((size_t)i * Wd + j);
+                    texels[(size_t)i * Wd + j] = make_float4(p[0], p[1], p[2], rows[(size_t)i * (Wd + 1) + j + 1]);
+                }
             const float4 *tp4;
             if ((st = upload(sc, texels.data(), texels.size(), &tp4)) != RT_OK) { rt_scene_destroy(sc); return st; }
-            D.env_rgb = tp4;
-            if ((st = upload(sc, rows.data(), rows.size(), &dp)) != RT_OK) { rt_scene_destroy(sc); return st; }
-            D.env_row_cdf = dp;
+            D.env_texel = tp4;
             if ((st = upload(sc, marg.c.data(), marg.c.size(), &dp)) != RT_OK) { rt_scene_destroy(sc); return st; }
             D.env_marginal = dp;
             if ((st = upload(sc, weight.data(), weight.size(), &dp)) != RT_OK) { rt_scene_destroy(sc); return st; }
@@ -2906,18 +2908,18 @@ static rt_status scene_create(rt_ctx *ctx, const rt_scene_desc *d, const ExtTree
     }
     const float *fp;
     {
-        std::vector<float4> rec(3 * (size_t)nt);
+        auto bits = [](int n) { int b = 1; while (b < 31 && n >> b) b++; return b; };   // of 0..n
+        const int nb = bits(d->n_bsdfs), nl = bits(d->n_lights);
+        S.ids = nb + nl + bits(d->n_meshes) <= 32 ? TriIds{nb, nl, nb + nl} : TriIds{0, 0, 0};
+        std::vector<float> rec(RT_TRI_REC * (size_t)nt);
         for (int t = 0; t < nt; t++) {
+            float *R = &rec[RT_TRI_REC * (size_t)t];
+            std::memcpy(R, &tri_v[9 * (size_t)t], 9 * sizeof(float));
             const int m = tri_mesh[t];
-            const int ids[3] = {m < d->n_meshes ? d->meshes[m].bsdf : -1, m < d->n_meshes ? d->meshes[m].light : -1, m};
-            for (int k = 0; k < 3; k++) {
-                const float *p = &tri_v[9 * (size_t)t + 3 * k];
-                float w;
-                std::memcpy(&w, &ids[k], 4);
-                rec[3 * (size_t)t + k] = make_float4(p[0], p[1], p[2], w);
-            }
+            const unsigned word = S.ids.pack(m, d->meshes[m].bsdf, d->meshes[m].light);
+            std::memcpy(R + 9, &word, sizeof(word));
         }
-        const float4 *rp;
+        const float *rp;
         if ((st = upload(sc, rec.data(), rec.size(), &rp)) != RT_OK) { rt_scene_destroy(sc); return st; }
         S.tri_rec = rp;
     }
@@ -3218,7 +3220,7 @@ rt_status rt_scene_refit(rt_ctx *ctx, rt_scene *sc, const float *vertices, const
     }
     const int sm = ctx->sm_count > 0 ? ctx->sm_count : 1;
     auto grid = [&](int64_t n) { return (int)std::max<int64_t>(1, std::min<int64_t>((n + 255) / 256, (int64_t)sm * 16)); };
-    k_refit_tris<<<grid(n_tris), 256, 0, st>>>(vd, nd_, sc->indices_dev, n_tris, const_cast<float4 *>(sc->S.tri_rec),
+    k_refit_tris<<<grid(n_tris), 256, 0, st>>>(vd, nd_, sc->indices_dev, n_tris, const_cast<float *>(sc->S.tri_rec),
                                                const_cast<float *>(sc->S.tri_n));
     k_refit_slots<<<grid(n_tris), 256, 0, st>>>(const_cast<float4 *>(sc->S.tri_slots), n_tris, sc->S.tri_rec);
     for (size_t l = 0; l + 1 < sc->level_off.size(); l++) {

@@ -10,6 +10,26 @@
 #include "rt_math.cuh"
 
 // ------------------------------------------------------------------ layout
+#define RT_TRI_REC 10   // floats of a triangle record (DevScene::tri_rec)
+// The last word of a triangle record: BSDF + 1 in the low bits, light + 1 in
+// the next, the mesh in the rest, in as many bits each as the scene's counts
+// take; the mesh alone (bsdf_bits 0) where they do not fit.
+struct TriIds {
+    int bsdf_bits, light_bits, mesh_shift;   // mesh_shift = bsdf_bits + light_bits
+    __host__ __device__ __forceinline__ int mesh(unsigned w) const { return (int)(w >> mesh_shift); }
+    __host__ __device__ __forceinline__ int bsdf(unsigned w) const { return (int)(w & ((1u << bsdf_bits) - 1)) - 1; }
+    __host__ __device__ __forceinline__ int light(unsigned w) const
+    {
+        return (int)((w >> bsdf_bits) & ((1u << light_bits) - 1)) - 1;
+    }
+    __host__ __forceinline__ unsigned pack(int m, int b, int l) const
+    {
+        if (!bsdf_bits) return (unsigned)m;
+        return (unsigned)m << mesh_shift | (unsigned)(l < 0 ? 0 : l + 1) << bsdf_bits |
+               (unsigned)(b < 0 ? 0 : b + 1);
+    }
+};
+
 struct DevMesh {
     int first_tri, n_tris, bsdf, light, interior, exterior;
     int cdf_off;      // offset of this mesh's area CDF (n_tris + 1 floats)
@@ -83,8 +103,12 @@ struct DevLight {
     // environment map
     int env_w, env_h;
     float env_scale;
-    const float4 *env_rgb;      // W*H texels (rgb, 0): one 16-byte load each
-    const float *env_row_cdf;   // H * (W + 1)
+    // W*H texels: rgb and, beside it, entry column + 1 of the row's CDF (entry 0
+    // is 0): one 16-byte load per texel, from the sector that the search for a
+    // column ends in, in no more memory than colours and CDF apart.  Colours in
+    // 12 bytes, the CDF apart: 1.31M-triangle frame 0.6 % slower, the batch of
+    // 12 jobs 1.1 %.
+    const float4 *env_texel;
     const float *env_marginal;  // H + 1
     const float *env_weight;    // H
     const int *env_marg_guide;  // env_gm + 1 entries (cdf_guide of env_marginal)
@@ -140,13 +164,12 @@ struct DevScene {
     const float4 *wtri;
     int n_wnodes;
     // original geometry
-    // 3 float4 per triangle: (p0, BSDF), (p1, light), (p2, mesh), the indices
-    // as int bits (-1: none).  A hit's vertices, BSDF and light are three
-    // 16-byte loads side by side; as nine floats, a mesh index and the mesh's
-    // record they were a dozen loads in a chain of three (grid-medium frame, which
-    // asks for the BSDF of every boundary crossed, 49.0 -> 48.0 ms; the
-    // 1.31M-triangle frame 0.4 % faster).
-    const float4 *tri_rec;
+    // RT_TRI_REC floats per triangle: p0, p1, p2 and its mesh, light and BSDF
+    // (TriIds), five 8-byte loads side by side for a hit.  (With BSDF and light
+    // looked up in the mesh, a chain of loads more, the batch of 12 jobs was
+    // 0.9 % slower.)
+    const float *tri_rec;
+    TriIds ids;
     const float *tri_n;         // 9 floats per triangle (n0, n1, n2) or null
     const uint8_t *tri_type;    // queue code (bsdf_code_of) of the triangle's mesh BSDF, 255 = no BSDF
     const float *tri_uv;        // 6 floats per triangle (uv0, uv1, uv2) or null; NaN: mesh without uvs
@@ -441,12 +464,35 @@ __device__ __forceinline__ bool trace_ray(const DevScene &S, V3 o, V3 d, float m
 }
 
 // the nine vertex coordinates of a triangle record (DevScene::tri_rec)
-__device__ __forceinline__ void tri_load(const float4 *tri_rec, int t, float *P)
+__device__ __forceinline__ void tri_load(const float *tri_rec, int t, float *P)
 {
-    for (int k = 0; k < 3; k++) {
-        const float4 v = tri_rec[3 * (size_t)t + k];
-        P[3 * k] = v.x; P[3 * k + 1] = v.y; P[3 * k + 2] = v.z;
+    const float2 *R = reinterpret_cast<const float2 *>(tri_rec + RT_TRI_REC * (size_t)t);
+    for (int k = 0; k < 4; k++) {
+        const float2 v = R[k];
+        P[2 * k] = v.x; P[2 * k + 1] = v.y;
     }
+    P[8] = R[4].x;
+}
+// its vertices and last word
+__device__ __forceinline__ void tri_load(const float *tri_rec, int t, V3 &p0, V3 &p1, V3 &p2, unsigned &word)
+{
+    const float2 *R = reinterpret_cast<const float2 *>(tri_rec + RT_TRI_REC * (size_t)t);
+    const float2 a = __ldg(R), b = __ldg(R + 1), c = __ldg(R + 2), d = __ldg(R + 3), e = __ldg(R + 4);
+    p0 = v3(a.x, a.y, b.x); p1 = v3(b.y, c.x, c.y); p2 = v3(d.x, d.y, e.x);
+    word = __float_as_uint(e.y);
+}
+
+__device__ __forceinline__ unsigned tri_word(const DevScene &S, int t)
+{
+    return __float_as_uint(__ldg(&S.tri_rec[RT_TRI_REC * (size_t)t + 9]));
+}
+__device__ __forceinline__ int tri_bsdf(const DevScene &S, unsigned word)
+{
+    return S.ids.bsdf_bits ? S.ids.bsdf(word) : __ldg(&S.meshes[word].bsdf);
+}
+__device__ __forceinline__ int tri_light(const DevScene &S, unsigned word)
+{
+    return S.ids.bsdf_bits ? S.ids.light(word) : __ldg(&S.meshes[word].light);
 }
 
 // DifferentialGeometry::coordinateSystem (core/DifferentialGeometry.h:36-50)
@@ -471,11 +517,11 @@ __device__ __forceinline__ Frame hit_frame(const DevScene &S, const Hit &h, V3 o
 {
     Frame f;
     if (h.prim >= 0) {
-        const float4 *R = S.tri_rec + 3 * (size_t)h.prim;
-        const float4 r0 = __ldg(R), r1 = __ldg(R + 1), r2 = __ldg(R + 2);
-        bsdf = __float_as_int(r0.w);
-        light = __float_as_int(r1.w);
-        V3 p0 = v3(r0.x, r0.y, r0.z), p1 = v3(r1.x, r1.y, r1.z), p2 = v3(r2.x, r2.y, r2.z);
+        V3 p0, p1, p2;
+        unsigned word;
+        tri_load(S.tri_rec, h.prim, p0, p1, p2, word);
+        bsdf = tri_bsdf(S, word);
+        light = tri_light(S, word);
         float sum = h.u + h.v;
         float bx = 1 - sum;
         f.p = (bx * p0 + h.u * p1) + h.v * p2;
@@ -513,15 +559,15 @@ __device__ __forceinline__ V3 to_world(const Frame &f, V3 v) { return (f.s * v.x
 // primitive attributes
 __device__ __forceinline__ int prim_mesh(const DevScene &S, int prim)
 {
-    return __float_as_int(__ldg(&S.tri_rec[3 * (size_t)prim + 2].w));
+    return S.ids.mesh(tri_word(S, prim));
 }
 __device__ __forceinline__ int prim_bsdf(const DevScene &S, int prim)
 {
-    return prim >= 0 ? __float_as_int(__ldg(&S.tri_rec[3 * (size_t)prim].w)) : S.spheres[-prim - 2].bsdf;
+    return prim >= 0 ? __ldg(&S.meshes[prim_mesh(S, prim)].bsdf) : S.spheres[-prim - 2].bsdf;
 }
 __device__ __forceinline__ int prim_light(const DevScene &S, int prim)
 {
-    return prim >= 0 ? __float_as_int(__ldg(&S.tri_rec[3 * (size_t)prim + 1].w)) : S.spheres[-prim - 2].light;
+    return prim >= 0 ? __ldg(&S.meshes[prim_mesh(S, prim)].light) : S.spheres[-prim - 2].light;
 }
 // queue code (bsdf_code_of) of a hit primitive's BSDF, or -1 without a BSDF
 __device__ __forceinline__ int prim_type(const DevScene &S, int prim)
@@ -553,18 +599,28 @@ __device__ __forceinline__ int cdf_sample(const float *cdf, int n /* entries inc
     }
     return imin(imax(0, lo - 1), n - 2);
 }
+// CDFs that cdf_sample_guided searches
+struct PlainCdf {
+    const float *c;
+    __device__ __forceinline__ float operator[](int i) const { return __ldg(c + i); }
+};
+struct EnvRowCdf {   // of one row of DevLight::env_texel
+    const float4 *texel;
+    __device__ __forceinline__ float operator[](int i) const { return i > 0 ? __ldg(&texel[i - 1].w) : 0.f; }
+};
 // The same index as cdf_sample, with the search narrowed by a guide table:
 // guide[k] = first i with cdf[i] >= k / G (G a power of two, so k = (int)(u*G)
 // is exact).  For u in [k/G, (k+1)/G) the answer lies in [guide[k],
 // guide[k+1]], so a binary search over that range returns exactly what the
 // full lower_bound returns, in a step or two instead of log2(n).
-__device__ __forceinline__ int cdf_sample_guided(const float *cdf, int n, float u, const int *guide, int G)
+template <typename Cdf>
+__device__ __forceinline__ int cdf_sample_guided(Cdf cdf, int n, float u, const int *guide, int G)
 {
     int k = imin(imax((int)(u * (float)G), 0), G - 1);
     int lo = __ldg(guide + k), hi = __ldg(guide + k + 1);
     while (lo < hi) {
         int mid = lo + ((hi - lo) >> 1);
-        if (__ldg(cdf + mid) < u) lo = mid + 1; else hi = mid;
+        if (cdf[mid] < u) lo = mid + 1; else hi = mid;
     }
     return imin(imax(0, lo - 1), n - 2);
 }
@@ -1442,9 +1498,8 @@ struct LightRec {
 
 __device__ __forceinline__ void tri_verts(const DevScene &S, int tri, V3 &p0, V3 &p1, V3 &p2)
 {
-    const float4 *R = S.tri_rec + 3 * (size_t)tri;
-    const float4 r0 = __ldg(R), r1 = __ldg(R + 1), r2 = __ldg(R + 2);
-    p0 = v3(r0.x, r0.y, r0.z); p1 = v3(r1.x, r1.y, r1.z); p2 = v3(r2.x, r2.y, r2.z);
+    unsigned word;
+    tri_load(S.tri_rec, tri, p0, p1, p2, word);
 }
 
 // Mesh::sample (geometricShape/Mesh.cpp:38-68) + Triangle::sample (Triangle.cpp:251-273)
@@ -1547,10 +1602,10 @@ __device__ __forceinline__ C3 env_interp(const DevLight &L, float x, float y)
     int x0 = iclamp((int)x, 0, W - 2), y0 = iclamp((int)y, 0, H - 2);
     int x1 = x0 + 1 < W ? x0 + 1 : x0; x1 = iclamp(x1, 0, W - 1);
     int y1 = y0 + 1 < H ? y0 + 1 : y0; y1 = iclamp(y1, 0, H - 1);
-    const float4 a00 = __ldg(L.env_rgb + ((size_t)y0 * W + x0));
-    const float4 a01 = __ldg(L.env_rgb + ((size_t)y1 * W + x0));
-    const float4 a10 = __ldg(L.env_rgb + ((size_t)y0 * W + x1));
-    const float4 a11 = __ldg(L.env_rgb + ((size_t)y1 * W + x1));
+    const float4 a00 = __ldg(L.env_texel + ((size_t)y0 * W + x0));
+    const float4 a01 = __ldg(L.env_texel + ((size_t)y1 * W + x0));
+    const float4 a10 = __ldg(L.env_texel + ((size_t)y0 * W + x1));
+    const float4 a11 = __ldg(L.env_texel + ((size_t)y1 * W + x1));
     float w00 = (1 - ax) * (1 - ay), w01 = (1 - ax) * ay, w10 = ax * (1 - ay), w11 = ax * ay;
     C3 r;
     r.r = ((w00 * a00.x + w01 * a01.x) + w10 * a10.x) + w11 * a11.x;
@@ -1576,8 +1631,8 @@ __device__ __forceinline__ C3 env_le(const DevLight &L, V3 direction)
 __device__ __forceinline__ void env_sample(const DevLight &L, V3 p, V2 s, LightRec &o)
 {
     int W = L.env_w, H = L.env_h;
-    int row = cdf_sample_guided(L.env_marginal, H + 1, s.x, L.env_marg_guide, L.env_gm);
-    int col = cdf_sample_guided(L.env_row_cdf + (size_t)row * (W + 1), W + 1, s.y,
+    int row = cdf_sample_guided(PlainCdf{L.env_marginal}, H + 1, s.x, L.env_marg_guide, L.env_gm);
+    int col = cdf_sample_guided(EnvRowCdf{L.env_texel + (size_t)row * W}, W + 1, s.y,
                                 L.env_row_guide + (size_t)row * (L.env_gr + 1), L.env_gr);
     float rcol = (float)col + 0.f * (float)W;
     float rrow = (float)row + 0.f * (float)H;
@@ -1595,7 +1650,7 @@ __device__ __forceinline__ void env_sample(const DevLight &L, V3 p, V2 s, LightR
     o.point = p + L.env_radius * dir;
     o.normal = v3(0, 0, 0);
     int cx = iclamp(col, 0, W - 1), cy = iclamp(row, 0, H - 1);
-    const float4 texel = __ldg(L.env_rgb + ((size_t)cy * W + cx));
+    const float4 texel = __ldg(L.env_texel + ((size_t)cy * W + cx));
     o.intensity = c3(texel.x, texel.y, texel.z) * L.env_scale;
     float pdf = lum(o.intensity) * L.env_weight[row];
     float den = L.env_marginal_sum * (2 * RT_PI / (float)W);

@@ -40,7 +40,7 @@ __device__ __forceinline__ unsigned lbvh_expand10(unsigned v)
     return v;
 }
 
-__global__ void k_lbvh_codes(const float4 *tri_rec, int n, float bx0, float by0, float bz0, float sx, float sy, float sz,
+__global__ void k_lbvh_codes(const float *tri_rec, int n, float bx0, float by0, float bz0, float sx, float sy, float sz,
                              unsigned *codes, int *ids)
 {
     for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
@@ -191,7 +191,7 @@ __global__ void k_lbvh_nodes(const unsigned *codes, int n, float4 *nodes, int *i
 
 // boxes from the leaves up: every leaf writes its triangle's box into its
 // parent's child slot; the second arrival at a node unites the two and goes on
-__global__ void k_lbvh_boxes(const float4 *tri_rec, const int *ids, int n, const int *iparent, const int *lparent,
+__global__ void k_lbvh_boxes(const float *tri_rec, const int *ids, int n, const int *iparent, const int *lparent,
                              int *arrivals, float *boxes, int *max_depth)
 {
     for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < n; s += gridDim.x * blockDim.x) {
@@ -232,7 +232,7 @@ __global__ void k_lbvh_boxes(const float4 *tri_rec, const int *ids, int n, const
 }
 
 // triangle slots in sorted order: (p0, id), (p1 - p0), (p2 - p0)
-__global__ void k_lbvh_slots(const float4 *tri_rec, const int *ids, int n, float4 *slots)
+__global__ void k_lbvh_slots(const float *tri_rec, const int *ids, int n, float4 *slots)
 {
     for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < n; s += gridDim.x * blockDim.x) {
         const int id = ids[s];
