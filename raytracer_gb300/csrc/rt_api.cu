@@ -1662,106 +1662,195 @@ __global__ void k_film_multi(RenderParams P)
 // tile's screen holds its pixels plus an overlap of ceil(r - 0.5) pixels on
 // every side; samples splat value * w and w into every pixel of that screen
 // within the filter radius, w read from the 32 x 32 table; screens are merged
-// into the full screen in tile order.  One warp per output pixel gathers,
-// tile by tile in raster order (the merge order of a single-threaded run), the
-// samples of the tile's pixels that reach it, in the tile loop's pixel and
-// sample order.  k_film_jitter writes each sample's film position (from its
-// path stream) beside its radiance first, where the ended path's throughput
-// was, so that the gather reads one record per sample and pixel.  With the
-// stream seeded again for each of them, and pixels visited up to ceil(r + 0.5)
-// away, a 301x203 x 25 spp frame under a Gaussian of radius 2 took 1.25 ms;
-// now 0.30 ms.  A warp weighs 32 samples at a time and sums them in order; a
-// thread per pixel summing as it went took 0.60 ms (12 warps per SM, each
-// waiting on its one chain of adds and records).  The
+// into the full screen in tile order.  An output pixel gathers, tile by tile in
+// raster order (the merge order of a single-threaded run), the samples of the
+// tile's pixels that reach it, in the tile loop's pixel and sample order.  The
 // output is the full screen's top-left width x height block, which is what
 // the reference reads back (operator() and postProcessColor ignore the
 // overlap offset, Screen.h:52, Screen.cpp:113-122).
-__global__ void k_film_jitter(RenderParams P)
+//
+// Each sample's film position is drawn again from its path stream first.  Then
+// a thread per output pixel sums as it goes: radiance and position of sample s
+// of batch pixel q lie at s * npix + q (in the path state's rays and pending
+// samples, which ended paths no longer need), so that lanes on neighbouring
+// pixels read side by side.  On small films and at many samples (film_by_warp)
+// a warp per output pixel weighs 32 samples at a time and sums them in order:
+// the pixel's samples lie side by side as they are, their positions put beside
+// their radiance, where the ended path's throughput was.  Gaussian of radius 2,
+// 1024^2 x 16 spp: 2.05 ms by threads, 3.31 by warps (4.08 with every reader
+// drawing the positions for itself); 301x203 x 25 spp: 0.49, 0.30 (1.02).
+struct FilmSamples {
+    float4 *a;   // radiance, film x (infinite for a NaN sample, which reaches no pixel)
+    float *b;    // film y
+};
+__host__ __device__ __forceinline__ FilmSamples film_samples(const Wave &W)
 {
-    const int W = P.S.cam.width;
-    for (int slot = blockIdx.x * blockDim.x + threadIdx.x; slot < P.n_paths; slot += gridDim.x * blockDim.x) {
-        const int q = slot / P.spp, sm = slot - q * P.spp;
-        const int4 to = P.tileorder[P.g0 + q];
-        Pcg32 rng;
-        path_stream_seed(rng, P.seed, (uint32_t)(to.y * W + to.x), (uint32_t)(P.sample_begin + sm));
-        const V2 j = next2d(rng);
-        w_tp(P.W, slot) = make_float4((float)to.x + j.x, (float)to.y + j.y, 0.f, 0.f);
+    return {W.ray, reinterpret_cast<float *>(W.smp)};
+}
+// a sample's film position
+__device__ __forceinline__ V2 film_position(const RenderParams &P, int q, int s)
+{
+    const int4 to = P.tileorder[P.g0 + q];
+    Pcg32 rng;
+    path_stream_seed(rng, P.seed, (uint32_t)(to.y * P.S.cam.width + to.x), (uint32_t)(P.sample_begin + s));
+    const V2 j = next2d(rng);
+    return v2((float)to.x + j.x, (float)to.y + j.y);
+}
+__global__ void k_film_positions(RenderParams P)   // for a warp per pixel
+{
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < P.n_paths; i += gridDim.x * blockDim.x) {
+        const int q = i / P.spp;
+        const V2 at = film_position(P, q, i - q * P.spp);
+        w_tp(P.W, i) = make_float4(at.x, at.y, 0.f, 0.f);
     }
 }
-__global__ void __launch_bounds__(128) k_film_wide(RenderParams P, float4 *film, int t0, int t1, int tiles_x, int bx, int by)
+#define RT_FILM_RUN 8   // samples of a pixel per thread: a line or two of records
+__global__ void k_film_samples(RenderParams P)   // for a thread per pixel
 {
-    __shared__ float4 terms[4][4][8];   // per warp, channel: the terms of 32 samples
+    const FilmSamples F = film_samples(P.W);
+    const int runs = (P.spp + RT_FILM_RUN - 1) / RT_FILM_RUN;
+    for (int64_t i = blockIdx.x * blockDim.x + threadIdx.x; i < (int64_t)runs * P.npix; i += gridDim.x * blockDim.x) {
+        const int run = (int)(i / P.npix), q = (int)(i - (int64_t)run * P.npix);
+        const int s1 = imin(P.spp, (run + 1) * RT_FILM_RUN);
+        for (int s = run * RT_FILM_RUN; s < s1; s++) {
+            const float4 L = w_rad(P.W, q * P.spp + s);
+            const V2 p = film_position(P, q, s);
+            const size_t at = (size_t)s * P.npix + q;
+            F.a[at] = make_float4(L.x, L.y, L.z, isnan(L.x) || isnan(L.y) || isnan(L.z) ? INFINITY : p.x);
+            F.b[at] = p.y;
+        }
+    }
+}
+// The terms (value * w and w) of a sample of radiance L at (x, y) in the pixel
+// at (lx, ly) of a tile's screen with origin (x0, y0) on the film; false when it
+// does not reach it.
+__device__ __forceinline__ bool film_term(const DevCamera &cam, float4 L, float x, float y, float lx, float ly, float x0,
+                                          float y0, float4 &term)
+{
+    const float rx = cam.frx, ry = cam.fry;
+    const float xl = x - 0.5f - x0, yl = y - 0.5f - y0;
+    const int ix = imin((int)((32 * fabsf(lx - xl)) / rx), 31);
+    const int iy = imin((int)((32 * fabsf(ly - yl)) / ry), 31);
+    const float w = __ldg(cam.filter_table + ix + iy * 32);
+    term = make_float4(L.x * w, L.y * w, L.z * w, w);
+    return lx >= xl - rx && lx <= xl + rx && ly >= yl - ry && ly <= yl + ry;
+}
+// a sample lies within half a pixel of its pixel's centre; the slack covers
+// the rounding of film positions
+__host__ __device__ __forceinline__ int film_reach(float radius) { return (int)floorf(radius + 0.51f); }
+template <bool WARP>
+__global__ void __launch_bounds__(128) k_film_wide(RenderParams P, float4 *film, int t0, int t1, int tiles_x, int bx,
+                                                   int by)
+{
+    __shared__ float4 terms[WARP ? 4 : 1][4][8];   // per warp, channel: the terms of 32 samples
     const DevCamera &cam = P.S.cam;
     const int W = cam.width, H = cam.height;
     const int ovx = cam.ov_x, ovy = cam.ov_y;
-    const float rx = cam.frx, ry = cam.fry;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int i = blockIdx.x * 4 + warp;
+    const int lane = threadIdx.x & 31, warp = WARP ? threadIdx.x >> 5 : 0;
+    const int i = WARP ? blockIdx.x * 4 + warp : blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= W * H) return;
     float *term = reinterpret_cast<float *>(terms[warp]);
+    const FilmSamples F = film_samples(P.W);
     const int ax = i % W, ay = i / W;   // full-screen (overlapped) coordinates
-    // lanes 0-3 hold the pixel's channels
+    // WARP: lanes 0-3 hold the pixel's channels, in .x
     float *out = reinterpret_cast<float *>(film + i) + (lane & 3);
-    float acc = *out;
+    float4 acc = WARP ? make_float4(*out, 0.f, 0.f, 0.f) : film[i];
     const int ty_hi = imin((H + by - 1) / by - 1, ay / by), tx_hi = imin(tiles_x - 1, ax / bx);
     const int ty_lo = imax(0, (ay - 2 * ovy) / by - 1), tx_lo = imax(0, (ax - 2 * ovx) / bx - 1);
-    // a sample lies within half a pixel of its pixel's centre; the slack
-    // covers the rounding of film positions
-    const int reach_x = (int)floorf(rx + 0.51f), reach_y = (int)floorf(ry + 0.51f);
+    const int reach_x = film_reach(cam.frx), reach_y = film_reach(cam.fry);
     for (int ty = ty_lo; ty <= ty_hi; ty++) {
         const int oy = ty * by, th = imin(by, H - oy);
         for (int tx = tx_lo; tx <= tx_hi; tx++) {
             const int t = ty * tiles_x + tx;
             if (t < t0 || t >= t1) continue;
             const int ox = tx * bx, tw = imin(bx, W - ox);
-            const int lx = ax - ox, ly = ay - oy;
-            if (lx < 0 || ly < 0 || lx >= tw + 2 * ovx || ly >= th + 2 * ovy) continue;
+            if (ax < ox || ay < oy || ax >= ox + tw + 2 * ovx || ay >= oy + th + 2 * ovy) continue;
+            // position in the tile's screen, and the screen's origin on the film
+            const float lx = (float)(ax - ox), ly = (float)(ay - oy);
+            const float x0 = (float)(ox - ovx), y0 = (float)(oy - ovy);
             // first batch pixel of the tile: full tile rows above, then the tiles to the left
-            const int tile_first = oy * W + ox * th;
+            const int tile_first = oy * W + ox * th - P.g0;
             const int qx0 = imax(ox, ax - ovx - reach_x), qx1 = imin(ox + tw - 1, ax - ovx + reach_x);
             const int qy0 = imax(oy, ay - ovy - reach_y), qy1 = imin(oy + th - 1, ay - ovy + reach_y);
-            const int nx = qx1 - qx0 + 1, ny = qy1 - qy0 + 1;
-            if (nx <= 0 || ny <= 0) { acc += 0.f; continue; }
-            const int n = nx * ny * P.spp;
-            float sum = 0.f;
-            for (int base = 0; base < n; base += 32) {
-                // a sample per lane, in the tile loop's order
-                const int idx = base + lane;
-                float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-                if (idx < n) {
-                    const int pix = idx / P.spp, sm = idx - pix * P.spp;
-                    const int row = pix / nx;
-                    const int q = tile_first - P.g0 + (qy0 + row - oy) * tw + (qx0 + pix - row * nx - ox);
-                    const float4 *p = P.W.acc + 2 * ((size_t)q * P.spp + sm);
-                    const float4 at = __ldg(p), L = __ldg(p + 1);
-                    float xl = at.x - 0.5f - (float)(ox - ovx);
-                    float yl = at.y - 0.5f - (float)(oy - ovy);
-                    int sx = imax(0, (int)ceilf(xl - rx)), ex = imin(tw + 2 * ovx - 1, (int)floorf(xl + rx));
-                    int sy = imax(0, (int)ceilf(yl - ry)), ey = imin(th + 2 * ovy - 1, (int)floorf(yl + ry));
-                    if (lx >= sx && lx <= ex && ly >= sy && ly <= ey && !(isnan(L.x) || isnan(L.y) || isnan(L.z))) {
-                        int ix = imin((int)((32 * fabsf((float)lx - xl)) / rx), 31);
-                        int iy = imin((int)((32 * fabsf((float)ly - yl)) / ry), 31);
-                        float w = __ldg(cam.filter_table + ix + iy * 32);
-                        v = make_float4(L.x * w, L.y * w, L.z * w, w);
+            float4 sum = make_float4(0.f, 0.f, 0.f, 0.f), v;
+            if (!WARP) {
+                for (int qy = qy0; qy <= qy1; qy++)
+                    for (int qx = qx0; qx <= qx1; qx++) {
+                        size_t at = (size_t)(tile_first + (qy - oy) * tw + (qx - ox));
+#pragma unroll 4
+                        for (int s = 0; s < P.spp; s++, at += (size_t)P.npix) {
+                            const float4 L = __ldg(F.a + at);
+                            if (film_term(cam, L, L.w, __ldg(F.b + at), lx, ly, x0, y0, v)) {
+                                sum.x += v.x; sum.y += v.y; sum.z += v.z; sum.w += v.w;
+                            }
+                        }
                     }
-                }
-                __syncwarp();
-                term[lane] = v.x; term[32 + lane] = v.y; term[64 + lane] = v.z; term[96 + lane] = v.w;
-                __syncwarp();
-                // summed in order, a channel per lane (a sample that does not
-                // reach the pixel adds +0, which changes no sum that began at +0)
-                if (lane < 4) {
+            } else if (qx0 <= qx1 && qy0 <= qy1) {
+                const int nx = qx1 - qx0 + 1, n = nx * (qy1 - qy0 + 1) * P.spp;
+                for (int base = 0; base < n; base += 32) {
+                    // a sample per lane, in the tile loop's order
+                    // (one that does not reach the pixel adds +0, which changes no sum that began at +0)
+                    const int idx = base + lane;
+                    v = make_float4(0.f, 0.f, 0.f, 0.f);
+                    if (idx < n) {
+                        const int pix = idx / P.spp, row = pix / nx;
+                        const int q = tile_first + (qy0 + row - oy) * tw + (qx0 + pix - row * nx - ox);
+                        const float4 *p = P.W.acc + 2 * ((size_t)q * P.spp + (idx - pix * P.spp));
+                        const float4 at = __ldg(p), L = __ldg(p + 1);
+                        if (!film_term(cam, L, at.x, at.y, lx, ly, x0, y0, v) || isnan(L.x) || isnan(L.y) || isnan(L.z))
+                            v = make_float4(0.f, 0.f, 0.f, 0.f);
+                    }
+                    __syncwarp();
+                    term[lane] = v.x; term[32 + lane] = v.y; term[64 + lane] = v.z; term[96 + lane] = v.w;
+                    __syncwarp();
+                    // summed in order, a channel per lane
+                    if (lane < 4) {
 #pragma unroll
-                    for (int k = 0; k < 8; k++) {
-                        const float4 s4 = terms[warp][lane][k];
-                        sum += s4.x; sum += s4.y; sum += s4.z; sum += s4.w;
+                        for (int k = 0; k < 8; k++) {
+                            const float4 s4 = terms[warp][lane][k];
+                            sum.x += s4.x; sum.x += s4.y; sum.x += s4.z; sum.x += s4.w;
+                        }
                     }
                 }
             }
-            acc = acc + sum;
+            acc = make_float4(acc.x + sum.x, acc.y + sum.y, acc.z + sum.z, acc.w + sum.w);
         }
     }
-    if (lane < 4) *out = acc;
+    if (!WARP) film[i] = acc;
+    else if (lane < 4) *out = acc.x;
+}
+// Which form the film takes, by the output pixels that there are threads for
+// and the samples that a pixel weighs.  A thread per pixel leaves a small film's
+// chip empty; at many samples its reads, npix records apart, find nothing in
+// L1.  Milliseconds by warps / by threads, pixels x samples weighed:
+// 61k: 72 .070 / .071, 100 .082 / .084, 625 .30 / .49.  120k: 225 .27 / .24, 450
+// .48 / .54, 625 .57 / .60.  262k: 625 1.24 / .93, 1250 2.4 / 2.3, 2500 4.6 / 5.7.
+// 524k: 2500 9.2 / 10.1.  1.05M: 25 .64 / .18, 625 4.9 / 3.3, 1250 9.5 / 8.3.
+#ifndef RT_FILM_FORM
+#define RT_FILM_FORM 0   // (1: always a thread per pixel, 2: always a warp; for measurements)
+#endif
+static bool film_by_warp(const RenderParams &P, int sm)
+{
+    if (RT_FILM_FORM) return RT_FILM_FORM == 2;
+    const DevCamera &cam = P.S.cam;
+    const int64_t npix = (int64_t)cam.width * cam.height;
+    const int64_t weighed = (int64_t)(2 * film_reach(cam.frx) + 1) * (2 * film_reach(cam.fry) + 1) * P.spp;
+    if (npix < (int64_t)640 * sm) return weighed >= 96;
+    if (npix < (int64_t)1280 * sm) return weighed >= 450;
+    return weighed >= 1600 && P.spp >= 64;
+}
+static void launch_film_wide(const RenderParams &P, float4 *film, int t0, int t1, int tiles_x, int bx, int by, int sm,
+                             cudaStream_t st)
+{
+    const int64_t npix = (int64_t)P.S.cam.width * P.S.cam.height;
+    const int blocks = std::min((P.n_paths + 255) / 256, sm * 16);
+    if (film_by_warp(P, sm)) {
+        k_film_positions<<<blocks, 256, 0, st>>>(P);
+        k_film_wide<true><<<(int)((npix + 3) / 4), 128, 0, st>>>(P, film, t0, t1, tiles_x, bx, by);
+    } else {
+        k_film_samples<<<blocks, 256, 0, st>>>(P);
+        k_film_wide<false><<<(int)((npix + 127) / 128), 128, 0, st>>>(P, film, t0, t1, tiles_x, bx, by);
+    }
 }
 
 // ---------------------------------------------------------------- standalone queries
@@ -3377,7 +3466,6 @@ static rt_status pt_batch_graph(rt_ctx *ctx, rt_scene *sc, const RenderParams &P
     const int cam_blocks = std::min((P.n_paths + 255) / 256, sm * 16);
     const int trace_blocks = sm * ctx->trace_bpsm, shade_blocks = sm * ctx->shade_bpsm;
     const int width = trace_width(ctx, sc);
-    const size_t npix_all = (size_t)Wd * sc->S.cam.height;
     struct Tail {
         const void *film;
         int box, accumulate, wd, t0, t1, tiles_x, bx, by, max_rounds, round_buf, cam_blocks, trace_blocks,
@@ -3464,10 +3552,7 @@ static rt_status pt_batch_graph(rt_ctx *ctx, rt_scene *sc, const RenderParams &P
                 break;
             }
             if (box_film) k_film<<<(P.npix + 127) / 128, 128, 0, st>>>(P, film, Wd, accumulate);
-            else {
-                k_film_jitter<<<cam_blocks, 256, 0, st>>>(P);
-                k_film_wide<<<(int)((npix_all + 3) / 4), 128, 0, st>>>(P, film, t0, t1, tiles_x, bx, by);
-            }
+            else launch_film_wide(P, film, t0, t1, tiles_x, bx, by, sm, st);
             if (bad(cudaGetLastError(), "film kernel")) break;
         } while (0);
         if (body_capturing) {
@@ -3739,8 +3824,7 @@ rt_status rt_render(rt_ctx *ctx, rt_scene *sc, const rt_render_desc *rd, float *
             int fb = (P.npix + 127) / 128;
             k_film<<<fb, 128, 0, st>>>(P, film, Wd, accumulate);
         } else {
-            k_film_jitter<<<cam_blocks, 256, 0, st>>>(P);
-            k_film_wide<<<(int)((npix_all + 3) / 4), 128, 0, st>>>(P, film, t0, t1, tiles_x, bx, by);
+            launch_film_wide(P, film, t0, t1, tiles_x, bx, by, sm, st);
             launches++;
         }
         prof_end(ctx);
