@@ -307,7 +307,11 @@ __device__ __forceinline__ int hit_queue(const RenderParams &P, const DevScene &
 // closest-hit traversal on the 1.31M-triangle frame: the staging code spills
 // in the node loop, and the few lanes that fetch do not wait on the atomic
 // for long.)
-template <bool ANY>
+// QUERY: rays of rt_trace.  An any-hit one lies in its slot's ray record
+// alone and its answer in q_end[slot]: in the shadow-ray record, half of each
+// of two sectors was read and a sector written per answer (4M any-hit rays in
+// device memory 1.30 ms, now 1.23).
+template <bool ANY, bool QUERY>
 __device__ __forceinline__ int trace_fetch(const Wave &W, const int *queue, int *wc, int n, bool want, float4 &o, float4 &d)
 {
     const int lane = threadIdx.x & 31;
@@ -320,7 +324,7 @@ __device__ __forceinline__ int trace_fetch(const Wave &W, const int *queue, int 
     const int q = base + __popc(m & ((1u << lane) - 1));
     if (!want || q >= n) return -1;
     const int slot = queue[q];
-    if (ANY) {
+    if (ANY && !QUERY) {
         o = w_ray_o(W, slot);
         d = w_sh_d(W, slot);
     } else {
@@ -456,7 +460,7 @@ __global__ void k_sort_copy(RenderParams P, int round, int shadow)
 #endif
 // MULTI: a multi-scene batch; each ray traverses the tree of its path's
 // scene (P.scenes[W.sid[slot]]), held per lane
-template <bool ANY, bool COUNT, bool MULTI = false>
+template <bool ANY, bool COUNT, bool MULTI = false, bool QUERY = false>
 __global__ void __launch_bounds__(128, ANY ? RT_TRACE_MINB_ANY : RT_TRACE_MINB) k_trace(RenderParams P, int round)
 {
     round = cur_round(P, round);
@@ -506,7 +510,7 @@ __global__ void __launch_bounds__(128, ANY ? RT_TRACE_MINB_ANY : RT_TRACE_MINB) 
         // ---- fetch rays for lanes whose ray is finished
         const bool terminated = (node == RT_SENT);
         float4 o4, d4;
-        const int got = trace_fetch<ANY>(P.W, queue, wc, n, terminated, o4, d4);
+        const int got = trace_fetch<ANY, QUERY>(P.W, queue, wc, n, terminated, o4, d4);
         if (terminated) {
             has_ray = got >= 0;
             if (has_ray) {
@@ -603,7 +607,8 @@ __global__ void __launch_bounds__(128, ANY ? RT_TRACE_MINB_ANY : RT_TRACE_MINB) 
                     }
                 }
             }
-            if (ANY) w_set_occluded(P.W, slot, hprim != -1);
+            if (ANY && QUERY) P.W.q_end[slot] = hprim != -1;
+            else if (ANY) w_set_occluded(P.W, slot, hprim != -1);
             else {
                 if (hprim != -1) P.W.hit[slot] = make_float4(hit_t, hu, hv, __int_as_float(hprim));
                 to_queue = MULTI ? hit_queue(P, *ms, hprim, n) : hit_queue(P, S, hprim, n);
@@ -664,7 +669,7 @@ __device__ __forceinline__ int link4(const int4 &cc, unsigned key)
     return s == 0 ? cc.x : s == 1 ? cc.y : s == 2 ? cc.z : cc.w;
 }
 
-template <bool ANY, bool COUNT>
+template <bool ANY, bool COUNT, bool QUERY = false>
 __global__ void __launch_bounds__(128, RT_TRACE4_MINB) k_trace4(RenderParams P, int round)
 {
     round = cur_round(P, round);
@@ -692,7 +697,7 @@ __global__ void __launch_bounds__(128, RT_TRACE4_MINB) k_trace4(RenderParams P, 
         // ---- fetch rays for lanes whose ray is finished
         const bool terminated = (node == RT_SENT);
         float4 o4, d4;
-        const int got = trace_fetch<ANY>(P.W, queue, wc, n, terminated, o4, d4);
+        const int got = trace_fetch<ANY, QUERY>(P.W, queue, wc, n, terminated, o4, d4);
         if (terminated) {
             has_ray = got >= 0;
             if (has_ray) {
@@ -785,7 +790,8 @@ __global__ void __launch_bounds__(128, RT_TRACE4_MINB) k_trace4(RenderParams P, 
                     }
                 }
             }
-            if (ANY) w_set_occluded(P.W, slot, hprim != -1);
+            if (ANY && QUERY) P.W.q_end[slot] = hprim != -1;
+            else if (ANY) w_set_occluded(P.W, slot, hprim != -1);
             else {
                 if (hprim != -1) P.W.hit[slot] = make_float4(hit_t, hu, hv, __int_as_float(hprim));
                 to_queue = hit_queue(P, S, hprim, n);
@@ -833,7 +839,7 @@ __device__ __forceinline__ unsigned meta_byte(int4 w1, unsigned slot)
     return (w >> (8 * (slot & 3))) & 0xffu;
 }
 
-template <bool ANY, bool COUNT>
+template <bool ANY, bool COUNT, bool QUERY = false>
 __global__ void __launch_bounds__(128, 8) k_trace8(RenderParams P, int round)
 {
     round = cur_round(P, round);
@@ -864,7 +870,7 @@ __global__ void __launch_bounds__(128, 8) k_trace8(RenderParams P, int round)
         const bool idle = !trav;
         bool has_ray = trav;
         float4 o4, d4;
-        const int got = trace_fetch<ANY>(P.W, queue, wc, n, idle, o4, d4);
+        const int got = trace_fetch<ANY, QUERY>(P.W, queue, wc, n, idle, o4, d4);
         if (idle) {
             has_ray = got >= 0;
             if (has_ray) {
@@ -988,7 +994,8 @@ __global__ void __launch_bounds__(128, 8) k_trace8(RenderParams P, int round)
                     }
                 }
             }
-            if (ANY) w_set_occluded(P.W, slot, hprim != -1);
+            if (ANY && QUERY) P.W.q_end[slot] = hprim != -1;
+            else if (ANY) w_set_occluded(P.W, slot, hprim != -1);
             else {
                 if (hprim != -1) P.W.hit[slot] = make_float4(hit_t, hu, hv, __int_as_float(hprim));
                 to_queue = hit_queue(P, S, hprim, n);
@@ -1018,10 +1025,9 @@ __global__ void k_rays_in(const rt_ray *rays, int n, RenderParams P, int anyhit)
     if (i >= n) return;
     rt_ray r = rays[i];
     float4 o = make_float4(r.o[0], r.o[1], r.o[2], r.mint), d = make_float4(r.d[0], r.d[1], r.d[2], r.maxt);
-    w_ray_o(P.W, i) = o;
-    if (anyhit) { w_sh_d(P.W, i) = d; P.W.q_shadow[i] = i; }
+    w_store2(P.W.ray, i, o, d);
+    if (anyhit) P.W.q_shadow[i] = i;
     else {
-        w_ray_d(P.W, i) = d;
         P.W.hit[i] = make_float4(0.f, 0.f, 0.f, __int_as_float(-1));   // the trace writes hits only
         P.W.q_closest[i] = i;
     }
@@ -1039,7 +1045,7 @@ __global__ void k_hits_out(RenderParams P, int n, int anyhit, rt_hit *hits)
     if (i >= n) return;
     rt_hit h;
     if (anyhit) {
-        h.t = 0.f; h.u = 0.f; h.v = 0.f; h.prim = __float_as_int(w_nee(P.W, i).w) ? 0 : -1;
+        h.t = 0.f; h.u = 0.f; h.v = 0.f; h.prim = P.W.q_end[i] ? 0 : -1;
     } else {
         float4 v = P.W.hit[i];
         int prim = __float_as_int(v.w);
@@ -4364,7 +4370,11 @@ rt_status rt_trace(rt_ctx *ctx, rt_scene *sc, const rt_ray *rays, int32_t n, int
     const int sm = ctx->sm_count > 0 ? ctx->sm_count : 1;
     CK(cudaMemsetAsync(ctx->limit_flag, 0, sizeof(int), st));
     k_rays_in<<<(n + 127) / 128, 128, 0, st>>>(dr, n, P, anyhit ? 1 : 0);
-    launch_trace(trace_width(ctx, sc), P, 0, anyhit != 0, false, sm * 12, st);
+    const int width = trace_width(ctx, sc);
+    if (!anyhit) launch_trace(width, P, 0, false, false, sm * 12, st);
+    else if (width == 8) k_trace8<true, false, true><<<sm * 12, 128, 0, st>>>(P, 0);
+    else if (width == 4) k_trace4<true, false, true><<<sm * 12, 128, 0, st>>>(P, 0);
+    else k_trace<true, false, false, true><<<sm * 12, 128, 0, st>>>(P, 0);
     k_hits_out<<<(n + 127) / 128, 128, 0, st>>>(P, n, anyhit ? 1 : 0, dh);
     s = launch_check("rt_trace kernels");
     if (s == RT_OK && !on_device) {
