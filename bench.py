@@ -361,10 +361,9 @@ def run_gpu(args):
     scene.render(8, seed=99, film=film.data_ptr())
     cstats = ctx.stats()
     pre_launches = cstats["launches"]
-    # graph launches (--graphs 1) time the steps without per-kernel events;
-    # the kernel split then comes from as many kernel-by-kernel profiled
-    # steps after the timed region
-    ctx.set_profiling(0 if args.graphs else 1)
+    # the steps are timed as a program runs them, without per-kernel events;
+    # the kernel split comes from as many profiled steps after the timed region
+    ctx.set_profiling(0)
     ctx.set_graphs(args.graphs)
     clocks = ClockSampler(local)
     clocks.start()   # before the warm-up: its first rows arrive after a moment
@@ -384,27 +383,21 @@ def run_gpu(args):
         scene.render(spp, seed=1000 + k, sample_begin=sbase, film=film.data_ptr())
         st = ctx.stats()
         launches += st["launches"]
-        for key in ("trace_closest_ms", "trace_any_ms", "shade_ms", "resolve_ms", "sort_ms", "volpath_ms", "camera_ms",
-                    "film_ms",
-                    "closest_rays",
-                    "shadow_rays", "trace_closest_launches", "trace_any_launches", "paths", "nan_samples"):
+        for key in ("closest_rays", "shadow_rays", "paths", "nan_samples"):
             agg[key] = agg.get(key, 0) + st[key]
     e1.record(stream)
     torch.cuda.nvtx.range_pop()
     barrier()
     clocks.end()
     clk = clocks.stop()
-    if args.graphs:
-        ctx.set_graphs(0)
-        ctx.set_profiling(1)
-        eager = {}
-        for k in range(args.steps):
-            scene.render(spp, seed=1000 + k, sample_begin=sbase, film=film.data_ptr())
-            st = ctx.stats()
-            for key in ("trace_closest_ms", "trace_any_ms", "shade_ms", "resolve_ms", "sort_ms", "volpath_ms",
-                        "camera_ms", "film_ms", "trace_closest_launches", "trace_any_launches"):
-                eager[key] = eager.get(key, 0) + st[key]
-        agg.update(eager)
+    ctx.set_graphs(0)
+    ctx.set_profiling(1)
+    for k in range(args.steps):
+        scene.render(spp, seed=1000 + k, sample_begin=sbase, film=film.data_ptr())
+        st = ctx.stats()
+        for key in ("trace_closest_ms", "trace_any_ms", "shade_ms", "resolve_ms", "sort_ms", "volpath_ms", "camera_ms",
+                    "film_ms", "trace_closest_launches", "trace_any_launches"):
+            agg[key] = agg.get(key, 0) + st[key]
     dev_ms = e0.elapsed_time(e1)
     t_local = dev_ms / 1000.0
     if world > 1:
@@ -536,8 +529,7 @@ def run_gpu(args):
                                      "(dependent node fetches, divergent lanes)"},
                 "mrays_per_s": rays_per_s / 1e6,
                 "kernel_ms": {k: round(v / args.steps, 3) for k, v in kern.items()},
-                "kernel_ms_source": ("kernel-by-kernel profiled steps after the graph-launched timed region"
-                                     if args.graphs else "CUDA events in the timed region"),
+                "kernel_ms_source": "CUDA events of the same steps, profiled after the timed region",
                 "traversal": {"nodes_per_closest_ray": nodes_pr_c, "tris_per_closest_ray": tris_pr_c,
                               "nodes_per_shadow_ray": nodes_pr_a, "tris_per_shadow_ray": tris_pr_a},
                 "gpu_launches": launches, "launches_before_timed": pre_launches,

@@ -329,7 +329,7 @@ typedef struct rt_render_stats {
     double trace_closest_ms; /* filled when profiling is enabled                 */
     double trace_any_ms;
     double shade_ms;
-    double volpath_ms;
+    double volpath_ms;       /* all VolPathTracing kernels                       */
     double film_ms;
     int64_t paths;           /* path samples rendered                            */
     int64_t closest_rays;    /* closest-hit rays traced                          */
@@ -384,7 +384,11 @@ rt_status rt_render_stats_get(const rt_ctx *ctx, rt_render_stats *out);
 rt_status rt_render_paths(rt_ctx *ctx, rt_scene *scene, const rt_render_desc *rd,
                           const int32_t *pixels, const int32_t *samples, int32_t n, float *rgb);
 /* Profiling level of later renders: 0 off, 1 per-kernel CUDA-event timing,
- * 2 timing plus BVH traversal counters (slower; for roofline accounting). */
+ * 2 timing plus BVH traversal counters (slower; for roofline accounting).
+ * Profiled PathTracingMIS renders run every round in the wavefront's kernels,
+ * one kind of work each, without the kernel that otherwise runs a round of few
+ * paths to its end; so do VolPathTracing renders at level 2.  Films and ray
+ * counts are the same; a small frame takes longer. */
 rt_status rt_ctx_set_profiling(rt_ctx *ctx, int32_t level);
 /* Tree used by later renders and rt_trace: 2 (binary BVH, the default), 4
  * (4-wide BVH collapsed from the binary one, same boxes) or 8 (compressed

@@ -2175,13 +2175,14 @@ static void graph_cache_clear(rt_ctx *c)
 #endif
 // P.tail_paths and P.tail_host for a render over the tree of `width`.  The
 // tail kernels trace the binary tree, so renders over another tree (a tie may
-// name another triangle there) and counting renders (profiling level 2) have
-// none.
+// name another triangle there) have none.  Nor have counting renders (profiling
+// level 2) and timed PathTracingMIS renders (level 1), whose times are one kind
+// of work each: a tail kernel traces and shades.
 static rt_status tail_setup(rt_ctx *c, int width, bool volpath, RenderParams &P)
 {
     P.tail_paths = -1;
     P.tail_host = nullptr;
-    if (c->profiling >= 2 || (!volpath && width != 2)) return RT_OK;
+    if (c->profiling >= (volpath ? 2 : 1) || (!volpath && width != 2)) return RT_OK;
     if (!c->tail_host) {
         CK(cudaHostAlloc(&c->tail_host, 8 * sizeof(int), cudaHostAllocMapped));
         CK(cudaHostGetDevicePointer(&c->tail_host_dev, c->tail_host, 0));
@@ -2211,7 +2212,7 @@ static rt_status tail_left(rt_ctx *c, const RenderParams &P, int r, int &left)
 
 // kinds for per-kernel timing
 enum { K_CAMERA = 0, K_TRACE_C = 1, K_TRACE_A = 2, K_SHADE = 3, K_VOLPATH = 4, K_FILM = 5, K_RESOLVE = 6, K_SORT = 7,
-       K_TAIL = 8, K_KINDS = 9 };
+       K_KINDS = 8 };
 
 static void prof_begin(rt_ctx *c, int kind)
 {
@@ -3781,9 +3782,7 @@ rt_status rt_render(rt_ctx *ctx, rt_scene *sc, const rt_render_desc *rd, float *
                 int ri = r;
                 const bool cnt2 = ctx->profiling >= 2;
                 if (tail && (r > 0 || P.n_paths <= P.tail_paths)) {
-                    prof_begin(ctx, K_TAIL);
                     launch_pt_tail(P, r, sm, st);
-                    prof_end(ctx);
                     launches++;
                     if ((s = launch_check("k_pt_tail")) != RT_OK || (s = tail_mark(ctx, P, r)) != RT_OK) return s;
                     if (r == 0) break;
@@ -3849,7 +3848,7 @@ rt_status rt_render(rt_ctx *ctx, rt_scene *sc, const rt_render_desc *rd, float *
     cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1);
     std::memset(&ctx->last, 0, sizeof(ctx->last));
     ctx->last.kernel_ms = ms;
-    double kt[K_KINDS] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+    double kt[K_KINDS] = {0, 0, 0, 0, 0, 0, 0, 0};
     for (size_t i = 0; i < ctx->ev_used; i++) {
         float e = 0.f;
         cudaEventElapsedTime(&e, ctx->ev_pool[2 * i], ctx->ev_pool[2 * i + 1]);
@@ -3858,7 +3857,7 @@ rt_status rt_render(rt_ctx *ctx, rt_scene *sc, const rt_render_desc *rd, float *
     ctx->last.camera_ms = kt[K_CAMERA];
     ctx->last.trace_closest_ms = kt[K_TRACE_C];
     ctx->last.trace_any_ms = kt[K_TRACE_A];
-    ctx->last.shade_ms = kt[K_SHADE] + kt[K_RESOLVE] + kt[K_TAIL];
+    ctx->last.shade_ms = kt[K_SHADE] + kt[K_RESOLVE];
     ctx->last.resolve_ms = kt[K_RESOLVE];
     ctx->last.sort_ms = kt[K_SORT];
     ctx->last.volpath_ms = kt[K_VOLPATH];
@@ -4119,9 +4118,7 @@ rt_status rt_internal_render_multi(rt_ctx *ctx, rt_scene *const *scenes, const r
         if ((s = launch_check("k_camera_multi")) != RT_OK) { release(); return s; }
         for (int r = 0; r < max_rounds; r++) {
             if (tail && (r > 0 || P.n_paths <= P.tail_paths)) {
-                prof_begin(ctx, K_TAIL);
                 launch_pt_tail(P, r, sm, st);
-                prof_end(ctx);
                 launches++;
                 if ((s = launch_check("k_pt_tail")) != RT_OK || (s = tail_mark(ctx, P, r)) != RT_OK) { release(); return s; }
                 if (r == 0) break;
@@ -4182,7 +4179,7 @@ rt_status rt_internal_render_multi(rt_ctx *ctx, rt_scene *const *scenes, const r
     cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1);
     std::memset(&ctx->last, 0, sizeof(ctx->last));
     ctx->last.kernel_ms = ms;
-    double kt[K_KINDS] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+    double kt[K_KINDS] = {0, 0, 0, 0, 0, 0, 0, 0};
     for (size_t i = 0; i < ctx->ev_used; i++) {
         float e = 0.f;
         cudaEventElapsedTime(&e, ctx->ev_pool[2 * i], ctx->ev_pool[2 * i + 1]);
@@ -4191,7 +4188,7 @@ rt_status rt_internal_render_multi(rt_ctx *ctx, rt_scene *const *scenes, const r
     ctx->last.camera_ms = kt[K_CAMERA];
     ctx->last.trace_closest_ms = kt[K_TRACE_C];
     ctx->last.trace_any_ms = kt[K_TRACE_A];
-    ctx->last.shade_ms = kt[K_SHADE] + kt[K_RESOLVE] + kt[K_TAIL];
+    ctx->last.shade_ms = kt[K_SHADE] + kt[K_RESOLVE];
     ctx->last.resolve_ms = kt[K_RESOLVE];
     ctx->last.film_ms = kt[K_FILM];
     ctx->last.trace_closest_launches = rounds_run;
