@@ -4513,6 +4513,31 @@ __global__ void k_tile_order(int4 *out, int ox, int oy, int tw, int th)
     out[i] = make_int4(ox + x, oy + y, x | (y << 16), tw | (th << 16));
 }
 
+// What a tile counts against the static scratch: 229 bytes per path (233 in
+// scenes that use the mixed queue), 17 per pixel, 64 per round, each array
+// rounded up to 256.  The line by which callers plan their tiles is fixed
+// here; the arrays carved now take 185 (189) bytes per path.
+static size_t static_tile_line(int64_t paths, int64_t npix, int rounds, bool mixed)
+{
+    size_t off = 0;
+    auto count = [&](size_t bytes, int arrays) {
+        for (int k = 0; k < arrays; k++) off = ((off + 255) & ~(size_t)255) + bytes;
+    };
+    count((size_t)paths * 16, 7);
+    count((size_t)paths * 4, 2);
+    count((size_t)paths * 16, 3);
+    count((size_t)paths * 4, 1);
+    count((size_t)paths * 16, 1);
+    count((size_t)paths, 1);
+    count((size_t)npix, 1);
+    count((size_t)paths * 4, 10 + mixed);
+    count((size_t)(rounds + 2) * 64, 1);
+    count((size_t)npix * 16, 1);
+    count((RT_STATIC_MAX_LIGHTS + 1) * 4, 1);
+    count(64, 1);
+    count(4, 2);
+    return off;
+}
 extern "C" rt_status rt_render_tile_static(rt_ctx *ctx, rt_scene *sc, const rt_render_desc *rd, int32_t tile_x,
                                            int32_t tile_y, float *film_rgbw_device)
 {
@@ -4598,34 +4623,12 @@ extern "C" rt_status rt_render_tile_static(rt_ctx *ctx, rt_scene *sc, const rt_r
     unsigned long long *stats = (unsigned long long *)take(8 * sizeof(unsigned long long));
     int *limit_flag = (int *)take(sizeof(int));
     int *work = (int *)take(sizeof(int));
-    // The requests that fit are those that fitted when the path state was
-    // one array per field (229 bytes per path and queue entries, about 15 %
-    // more than now): the line callers plan their tiles by stays.
-    {
-        size_t fields = 0;
-        auto count = [&](size_t bytes, int n) {
-            for (int k = 0; k < n; k++) fields = ((fields + 255) & ~(size_t)255) + bytes;
-        };
-        count(P * 16, 7);                                              // stream, ray and hit, throughput
-        count(P * 4, 2);
-        count(P * 16, 3);
-        count(P * 4, 1);
-        count(P * 16, 1);
-        count(P, 1);
-        count((size_t)npix, 1);
-        count(P * 4, 4 + RT_NBSDF + (sc->S.has_mixed ? 1 : 0));        // queues
-        count((size_t)(rounds + 2) * sizeof(RoundCounters), 1);
-        count((size_t)npix * sizeof(int4), 1);
-        count((size_t)(RT_STATIC_MAX_LIGHTS + 1) * sizeof(float), 1);
-        count(8 * sizeof(unsigned long long), 1);
-        count(sizeof(int), 2);
-        off = std::max(off, fields);
-    }
-    if (off > RT_STATIC_SCRATCH_BYTES) {
+    const size_t line = static_tile_line(paths, npix, rounds, sc->S.has_mixed != 0);
+    if (std::max(off, line) > RT_STATIC_SCRATCH_BYTES) {
         char msg[256];
         snprintf(msg, sizeof(msg),
-                 "rt_render_tile_static: a %dx%d tile at %d spp needs %zu bytes of path state; the static scratch "
-                 "holds %u (reduce spp or the block size)", tw, th, rd->spp, off, (unsigned)RT_STATIC_SCRATCH_BYTES);
+                 "rt_render_tile_static: a %dx%d tile at %d spp counts %zu bytes against the static scratch's %u "
+                 "(reduce spp or the block size)", tw, th, rd->spp, std::max(off, line), (unsigned)RT_STATIC_SCRATCH_BYTES);
         return fail(RT_ERR_LIMIT, msg);
     }
     cudaStream_t st = ctx->stream;

@@ -201,3 +201,26 @@ def test_static_tile_above_the_line_matches_oracle(ctx, rtlib, name):
     err = np.abs(got[..., :3] - ref[..., :3]) / np.maximum(np.abs(ref[..., :3]), 1e-3)
     assert np.mean(err.max(-1) > 1e-3) <= 0.22
     assert abs(got[..., :3].mean() / ref[..., :3].mean() - 1) <= 0.0075
+
+
+@pytest.mark.parametrize("make,size,spp", [(scenes.cornell_box, (32, 32), 143), (scenes.cornell_box, (20, 17), 430),
+                                           (scenes.cornell_box, (7, 5), 4185), (scenes.textured_room, (32, 32), 140),
+                                           (scenes.textured_room, (32, 8), 562)],
+                         ids=["32x32", "20x17", "7x5", "32x32_mixed", "32x8_mixed"])
+def test_static_tile_scratch_line(ctx, rtlib, make, size, spp):
+    """The most samples a tile may have under the static scratch's line, and
+    one more, whose refusal speaks of that line."""
+    torch = pytest.importorskip("torch")
+    w, h = size
+    g = rtlib.Scene(ctx, make(w, h))
+    film = torch.zeros((h, w, 4), dtype=torch.float32, device="cuda")
+    torch.cuda.synchronize()
+    try:
+        g.render_tile_static(0, 0, film.data_ptr(), spp, seed=6)
+        with pytest.raises(rtlib.RtError) as e:
+            g.render_tile_static(0, 0, film.data_ptr(), spp + 1, seed=6)
+        ref = g.render(spp, seed=6)
+    finally:
+        g.close()
+    assert e.value.status == 3 and "counts" in str(e.value) and "needs" not in str(e.value)
+    assert np.array_equal(film.cpu().numpy(), ref)
