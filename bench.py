@@ -160,7 +160,7 @@ def _config(data):
             "filter": getattr(_ARGS, "filter", "box"),
             "parallelism": "replicas" if int(os.environ.get("WORLD_SIZE", "1")) > 1 else "single",
             "l2": "inputs larger than L2: the scene (BVH, triangles, materials, maps) and the wavefront path "
-                  "state (218 bytes per path in flight, 314 for VolPathTracing) live in HBM"}
+                  "state (202 bytes per path in flight, 298 for VolPathTracing) live in HBM"}
 
 
 _ARGS = None
@@ -512,7 +512,7 @@ def run_gpu(args):
                            "sort_threshold": args.sort_threshold, "volpath_wavefront": args.volpath_wavefront,
                            "wave_paths": batch_paths},
                 "setup": {"scene_device_mb": round(info["device_bytes"] / 1e6, 1),
-                          "path_state_gb_per_batch": round(batch_paths * 205 / 1e9, 2),
+                          "path_state_gb_per_batch": round(batch_paths * (298 if CONFIG.get("volume") else 202) / 1e9, 2),
                           "scene_gen_s": round(gen_s, 2), "scene_build_upload_s": round(upload_s, 2)},
                 "e2e": None if args.small else {"value": e2e_value, "unit": UNIT, "h2d_bytes_per_step": h2d,
                                                 "d2h_bytes_per_step": d2h},

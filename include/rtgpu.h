@@ -408,7 +408,7 @@ enum { RT_BUILDER_HOST_SAH = 0, RT_BUILDER_DEVICE = 1 };
 rt_status rt_ctx_set_bvh_builder(rt_ctx *ctx, int32_t builder);
 /* Paths per wavefront batch of later renders (whole tiles x all samples are
  * batched up to this count): 2^16..2^26.  Device memory for path state is
- * about 240 bytes per path. */
+ * 202 bytes per path, 298 once a VolPathTracing render has run. */
 rt_status rt_ctx_set_wave_paths(rt_ctx *ctx, int32_t paths);
 /* Regroup the rays of every bounce after the first by direction octant and
  * origin cell before tracing them (0 off, 1 on); results are unchanged. */
@@ -469,8 +469,9 @@ rt_status rt_autotune(rt_ctx *ctx, rt_scene *const *scenes, const rt_render_desc
  * film_rgbw_device (a device pointer to the full width*height*4 film; only
  * the tile's pixels are written, or added to with RT_RENDER_ACCUMULATE),
  * with the same results as rt_render for those pixels.
- * Limits: tile pixels * spp * ~240 bytes of path state must fit the 32 MiB
- * static scratch (about 130k path samples, e.g. 32x32 at 128 spp);
+ * Limits: tile pixels * spp must fit the 32 MiB static scratch at 229 bytes
+ * per path sample (233 in scenes with textured or Microfacet BSDFs) and 17 per
+ * pixel: about 140k path samples, e.g. 32x32 at 128 spp;
  * PathTracingMIS max_depth <= 1024; at most 256 lights; larger requests
  * return RT_ERR_LIMIT.  The call synchronises the context's stream, so that
  * stream must not be under stream capture (RT_ERR_UNSUPPORTED otherwise).
@@ -541,10 +542,10 @@ typedef struct rt_job_info {
 } rt_job_info;
 rt_status rt_server_start(rt_ctx *ctx, const rt_server_opts *opts, rt_server **out);
 /* Device bytes of wavefront path state per path slot for an integrator
- * (RT_INTEGRATOR_*): the per-slot part of a render's working memory, and
- * what a server counts against its budget per slot (lanes at the
- * VolPathTracing figure, since a lane may take either kind of job).  0 for
- * an unknown integrator. */
+ * (RT_INTEGRATOR_*) as a server counts it against its budget (lanes at the
+ * VolPathTracing figure, since a lane may take either kind of job): a planning
+ * figure, 246 or 342, that renders stay below (rt_ctx_set_wave_paths).  0
+ * for an unknown integrator. */
 int64_t rt_path_state_bytes(int32_t integrator);
 /* Queue a render of `scene` (which must outlive the job).  A job whose
  * scene and films alone exceed the budget is refused (RT_ERR_LIMIT).

@@ -465,7 +465,7 @@ assert LIGHT_Q.itemsize == C.sizeof(D.LightQ) and LIGHT_R.itemsize == C.sizeof(D
 def path_state_bytes(integrator=0):
     """Device bytes of wavefront path state per path slot for an integrator
     (0: PathTracingMIS, 1: VolPathTracing), as a server counts them against
-    its budget."""
+    its budget (a planning figure; renders allocate less)."""
     return int(lib().rt_path_state_bytes(int(integrator)))
 
 

@@ -1060,7 +1060,7 @@ __global__ void k_hits_out(RenderParams P, int n, int anyhit, rt_hit *hits)
 // ---------------------------------------------------------------- PathTracingMIS vertex
 // The per-vertex loop body of PathTracingMIS::li (PathTracingMIS.cpp:54-259)
 // runs as three wavefront stages after the traces of a round:
-//   k_trace<closest>  sorts each traced path by what its ray hit (classify_hit);
+//   k_trace<closest>  sorts each traced path by what its ray hit (hit_queue);
 //   k_pt_finish       ends the paths whose ray missed or hit a surface without
 //                     a BSDF, and those that ended in shading with a light
 //                     sample pending: light sample if unoccluded (:140), the
@@ -1459,9 +1459,9 @@ __device__ __forceinline__ void tail_end(RoundCounters *C)
 // path, whatever their number; here the rounds that are left cost one launch
 // together.  The films are the wavefront's: the same functions run on the
 // same state, over the binary tree, whose two traversals meet their leaves in
-// the same order.  A 33-path rt_render_paths call 0.52 -> 0.11 ms, a 171x121 x
-// 4 spp preview with refit 1.79 -> 0.94 ms, Cornell 256^2 x 16 spp (its last
-// rounds) 1.44 -> 1.32 ms.  Bound by the latency of one path's chain of loads;
+// the same order.  A 33-path rt_render_paths call 0.45 -> 0.094 ms (its
+// staging kept by the context included), a 171x121 x 4 spp preview with refit
+// 1.72 -> 0.93, Cornell 256^2 x 16 spp (its last rounds) 1.44 -> 1.32.  Bound by the latency of one path's chain of loads;
 // two blocks per SM hold RT_PT_TAIL paths (3 to 8 blocks were 0-4 % slower).
 #ifndef RT_PT_TAIL_MINB
 #define RT_PT_TAIL_MINB 2
@@ -3381,11 +3381,11 @@ static rt_status ensure_vw(rt_ctx *c, int capacity)
     return RT_OK;
 }
 
-// What a server budgets per slot: the fields of the path state, each counted
-// by itself.  The arrays of ensure_wave and (VolPathTracing) ensure_vw take 28
-// bytes less (the shadow ray's origin, the eta of the pending sample and half
-// of the stream's increment are not stored); the figure stays, so that what a
-// budget admits does.
+// What a server budgets per slot, a planning figure that stays: the fields of
+// the path state, each counted by itself.  The arrays of ensure_wave take 202
+// bytes per slot, with ensure_vw's (VolPathTracing) 298: 44 less, since the final
+// radiance, the shadow ray's origin, the eta of the pending sample, the flags
+// and the occlusion lie inside other fields' records.
 extern "C" int64_t rt_path_state_bytes(int32_t integrator)
 {
     if (integrator != RT_INTEGRATOR_PATH_MIS && integrator != RT_INTEGRATOR_VOLPATH) return 0;

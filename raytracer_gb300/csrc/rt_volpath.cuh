@@ -504,7 +504,7 @@ __device__ __forceinline__ int *vw_trace_queue(const RenderParams &P, int round)
 __device__ __forceinline__ unsigned vw_step_path(const RenderParams &P, const DevScene &S, int slot, int &limit)
 {
     unsigned want = 0;
-    // ---- the trace (k_vw_trace)
+    // ---- the trace
     int flags;
     Pcg32 rng = path_rng(w_rng(P.W, slot), flags);
     const float4 ro = w_ray_o(P.W, slot), rd = w_ray_d(P.W, slot);
@@ -536,7 +536,7 @@ __device__ __forceinline__ unsigned vw_step_path(const RenderParams &P, const De
         flags = (flags & ~(VF_NULLX | VF_WAS)) | (was ? VF_WAS : 0);
         P.W.hit[slot] = make_float4(h.t, h.u, h.v, __int_as_float(h.prim));
     }
-    // ---- the step (k_vw_step)
+    // ---- the step
     C3 L = rgb(radv), T = rgb(tpv);
     const int depth = __float_as_int(radv.w);
     bool push_shadow = false, push_sample = false, push_trace = false;
