@@ -57,9 +57,10 @@ def build(force=False, verbose=False, ptxas_info=False):
         obj = os.path.join(BUILD, s + ".o")
         objs.append(obj)
         if force or _stale(obj, [src] + hdrs):
-            # -split-compile=0: the kernels are optimised in parallel (one translation
-            # unit: 178 s one after another, 59 s on eight cores)
-            cmd = [NVCC, ARCH, "-O3", "-lineinfo", "-std=c++17", "-fmad=false", "-split-compile=0", "-Xcompiler", "-fPIC",
+            # no -split-compile: under it a kernel's code changes with edits to others
+            # and with the machine's thread count (the persistent VolPath kernel 5.3 or
+            # 6.3 ms, closest-hit spills 52 or 72 bytes; without it 4.9 ms and 32)
+            cmd = [NVCC, ARCH, "-O3", "-lineinfo", "-std=c++17", "-fmad=false", "-Xcompiler", "-fPIC",
                    "-Xcompiler", "-ffp-contract=off",
                    "-I", os.path.join(ROOT, "include"), "-c", src, "-o", obj]
             if ptxas_info:
